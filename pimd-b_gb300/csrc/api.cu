@@ -358,7 +358,7 @@ static void free_handle(pimdb_handle* h) {
     double* bufs[] = {h->s.x,   h->s.p,   h->s.f,   h->s.fphys, h->s.fx,   h->s.E,        h->s.V,
                       h->s.Vb,  h->s.scal, h->s.Vh, h->s.Vbh,  h->s.yf,   h->s.yb,       h->s.Wf,
                       h->s.Wb,  h->s.Et, h->s.rowR, h->s.rowC, h->d_C,  h->d_T,    h->d_rot,      h->d_red[0],
-                      h->d_red[1], h->d_stage, h->d_part, h->s.Vp};
+                      h->d_red[1], h->d_stage, h->d_part, h->s.Vp, h->s.epart};
     for (double* b : bufs)
         if (b) cudaFree(b);
     if (h->d_err) cudaFree(h->d_err);
@@ -445,6 +445,7 @@ extern "C" int pimdb_create(const pimdb_config* cfg, void* cuda_stream, pimdb_ha
         e = cudaMalloc((void**)&s.Vp, 2 * ((size_t)s.N + 1) * sizeof(double));
         if (e == cudaSuccess) e = cudaMemset(s.Vp, 0xff, 2 * ((size_t)s.N + 1) * sizeof(double));
     }
+    if (e == cudaSuccess && s.bosonic) e = alloc(&s.epart, kEstimatorDoubles);
     if (e == cudaSuccess) e = alloc(&h->d_cm, 3);
     if (e == cudaSuccess && s.bosonic && exchange_energy_doubles(s, h->D) > 0)
         e = alloc(&h->d_ework, exchange_energy_doubles(s, h->D));

@@ -1040,7 +1040,7 @@ static size_t batch_smem(int D, int maxN, int threads, int maxPnm) {
     const size_t solve = sizeof(double) * (2 * (size_t)(maxN + 1) + 32);
     const size_t xforces = sizeof(double) * 2 * (size_t)D * maxN;  // beads 1 and P for the exchange forces
     const size_t xforces32 = sizeof(float) * std::max(xforces_f32_floats(D, maxN), 4 * (size_t)(maxN + 1));
-    const size_t estim = sizeof(double) * ((size_t)maxN + 1 + 32);
+    const size_t estim = sizeof(double) * 32;
     const size_t nmlines = sizeof(double) * nw * 8 * (size_t)maxPnm;  // normal-mode lines, 8 P per warp
     return 3 * 32 * sizeof(double) +
            std::max(std::max(std::max(stage, est), std::max(solve, estim)),

@@ -725,9 +725,41 @@ __global__ void k_exch_forces(Sys s, int accumulate, int adjoint, double vb_bar)
     exch_force_row<D>(s, w, lane, accumulate, nullptr, adjoint, vb_bar, ((volatile int*)s.xflags)[kExchBandLast]);
 }
 
-__global__ void k_exch_estimators(Sys s, int nbeads) {
-    extern __shared__ double sh[];
-    estimators_block(s, nbeads, sh);
+// The estimators, rows spread over the GPU: each block writes its totals to
+// its slot of Sys::epart and the block that finishes last adds the slots in
+// order (no waiting; deterministic).  One warp per row at a time, 16 bytes
+// read per packed entry within the band.
+__global__ void __launch_bounds__(kEstimatorThreads) k_exch_estimators(Sys s, int nbeads) {
+    __shared__ double red[32];
+    __shared__ int is_last;
+    const int nw = kEstimatorThreads / 32, tid = threadIdx.x;
+    double pe, pn, diag = 0.0;
+    estimator_rows(s, blockIdx.x * nw + (tid >> 5), gridDim.x * nw, tid & 31,
+                   ((volatile int*)s.xflags)[kExchBandLast], pe, pn);
+    pe = block_sum(pe, red);
+    pn = block_sum(pn, red);
+    if (tid == 0) {
+        s.epart[2 * blockIdx.x] = pe;
+        s.epart[2 * blockIdx.x + 1] = pn;
+        __threadfence();
+        is_last = atomicAdd(&s.xflags[kExchRowsCount], 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    pe = pn = 0.0;
+    for (int k = tid; k < (int)gridDim.x; k += kEstimatorThreads) {
+        pe += ((volatile double*)s.epart)[2 * k];
+        pn += ((volatile double*)s.epart)[2 * k + 1];
+    }
+    for (int m = tid; m < s.N; m += kEstimatorThreads) diag += s.E[tri(m) + m];
+    pe = block_sum(pe, red);
+    pn = block_sum(pn, red);
+    diag = block_sum(diag, red);
+    if (tid == 0) {
+        estimator_scalars(s, nbeads, pe, pn, diag);
+        s.xflags[kExchRowsCount] = 0;
+    }
 }
 
 // Every exchange kernel takes the largest shared-memory carveout.  An SM runs
@@ -919,11 +951,8 @@ void launch_exchange_adjoint(const Sys& s, int D, double vb_bar, cudaStream_t st
 }
 
 void launch_exchange_estimators(const Sys& s, cudaStream_t st) {
-    const size_t smem = sizeof(double) * (size_t)(s.N + 1 + 32);
-    int t = ((s.N + 31) / 32) * 32;
-    t = t > 512 ? 512 : (t < 32 ? 32 : t);
-    opt_in_smem((const void*)k_exch_estimators, smem);
-    k_exch_estimators<<<1, t, smem, st>>>(s, s.P);
+    const int rows = kEstimatorThreads / 32;
+    k_exch_estimators<<<std::min((s.N + rows - 1) / rows, kEstimatorBlocks), kEstimatorThreads, 0, st>>>(s, s.P);
 }
 
 }  // namespace pimdb

@@ -588,36 +588,64 @@ __device__ inline void exch_force_row(const Sys& s, int w, int lane, int accumul
     }
 }
 // primEstimator (:250-279), getDistinctProbability (:222-229) and
-// getLongestProbability (:238-240); one block, evaluated on request.
-// `sh` holds N+1+32 doubles.
-__device__ inline void estimators_block(const Sys& s, int nbeads, double* sh) {
-    double* G = sh;             // N+1
-    double* red = sh + s.N + 1; // 32
+// getLongestProbability (:238-240), on request.  The reference evaluates
+// primEstimator by a recursion over levels, G[m] = sum_u (G[u] - E[m-1][u])
+// exp(-beta (E[m-1][u] + V[u] - V[m])) / m; solved for G[N] it is minus the
+// mean energy of the closed cycles,
+//   G[N] = - sum_{l,u} p[l][u] E[l][u],
+// with the probabilities p[l][u] = Wf[l][u] y_u R_l (u <= l) that
+// exch_force_row sums: every entry is independent, where the recursion is a
+// chain of N block reductions on one block (a whole pimdb_exchange call at
+// N = 777: 8.46 ms with the recursion, 0.35 ms with the sum).
+// Each particle is in exactly one cycle, so sum p (l - u + 1) = N; dividing
+// by that sum takes out the common rounding of R.
+//
+// The shares of the rows w0, w0 + nw, ... of one warp: this lane's part of
+// sum p E and of sum p (l - u + 1).  `band` as in exch_force_row.
+__device__ inline void estimator_rows(const Sys& s, int w0, int nw, int lane, int band, double& pe, double& pn) {
     const int N = s.N;
-    const double beta = s.beta_ex;
-    const int tid = threadIdx.x, bd = blockDim.x;
-    if (tid == 0) G[0] = 0.0;
-    __syncthreads();
-    for (int m = 1; m <= N; ++m) {
-        const double* row = s.E + tri(m - 1);
-        double lmin = 1.79769313486231570815e308;
-        for (int u = tid; u < m; u += bd) lmin = fmin(lmin, row[u] + s.V[u]);
-        const double shift = block_min(lmin, red);
-        double ls = 0.0;
-        for (int u = tid; u < m; u += bd) ls += (G[u] - row[u]) * exp(-beta * (row[u] + s.V[u] - shift));
-        const double tot = block_sum(ls, red);
-        if (tid == 0) G[m] = tot / (m * exp(-beta * (s.V[m] - shift)));
-        __syncthreads();
+    const double beta = s.beta_ex, VN = s.V[N];
+    const bool exact = s.xflags[0] != 0;
+    pe = pn = 0.0;
+    for (int l = w0; l < N; l += nw) {
+        const size_t r = tri(l);
+        const double Rl = s.rowR[l], vbl = s.Vb[l + 1];
+        const int n0 = (band > 0 && !exact) ? max(0, l + 1 - band) / 32 * 32 : 0;
+        double re = 0.0, rn = 0.0, len = (double)(l + 1 - n0 - lane);
+        for (int n = n0 + lane; n <= l; n += 32, len -= 32.0) {
+            const double E = s.E[r + n];
+            double pr;
+            if (exact) {
+                pr = exp(-beta * (s.V[n] + E + vbl - VN)) / (l + 1);
+            } else {
+                const double w = s.Wf[r + n];
+                if (w == 0.0) continue;  // a cycle too costly to contribute adds exactly 0
+                pr = w * s.yf[n];
+            }
+            re = fma(pr, E, re);
+            rn = fma(pr, len, rn);
+        }
+        pe = fma(re, exact ? 1.0 : Rl, pe);
+        pn = fma(rn, exact ? 1.0 : Rl, pn);
     }
-    double diag = 0.0;
-    for (int m = tid; m < N; m += bd) diag += s.E[tri(m) + m];
+}
+// The scalars from the totals of the rows and sum_m E[m][m] (one thread).
+__device__ inline void estimator_scalars(const Sys& s, int nbeads, double pe, double pn, double diag) {
+    const int N = s.N;
+    const double beta = s.beta_ex, VN = s.V[N];
+    s.scal[1] = -(pe / pn) * N / nbeads;
+    s.scal[2] = exp(-beta * (diag - VN) - lgamma((double)(N + 1)));
+    s.scal[3] = exp(-beta * (s.E[tri(N - 1)] - VN));
+}
+// All of it by one block; `red` holds 32 doubles.
+__device__ inline void estimators_block(const Sys& s, int nbeads, double* red) {
+    double pe, pn, diag = 0.0;
+    estimator_rows(s, threadIdx.x >> 5, blockDim.x >> 5, threadIdx.x & 31, 0, pe, pn);
+    for (int m = threadIdx.x; m < s.N; m += blockDim.x) diag += s.E[tri(m) + m];
+    pe = block_sum(pe, red);
+    pn = block_sum(pn, red);
     diag = block_sum(diag, red);
-    if (tid == 0) {
-        const double VN = s.V[N];
-        s.scal[1] = G[N] / nbeads;
-        s.scal[2] = exp(-beta * (diag - VN) - lgamma((double)(N + 1)));
-        s.scal[3] = exp(-beta * (s.E[tri(N - 1)] - VN));
-    }
+    if (threadIdx.x == 0) estimator_scalars(s, nbeads, pe, pn, diag);
 }
 
 }  // namespace pimdb

@@ -102,7 +102,8 @@ constexpr int kExchBandDone = 14;
 // the entries beyond it, all exact zeros.
 constexpr int kExchBandLast = 15;
 // Index in Sys::xflags of the count of finished blocks of the per-row energy
-// kernel (its last block runs a due FP32 estimate).
+// kernel (its last block runs a due FP32 estimate) and of the estimators' (its
+// last block forms the scalars); 0 between launches.
 constexpr int kExchRowsCount = 9;
 // The banded solve: weights within kBandMax levels of the diagonal, one CTA
 // of kBandThreads per direction, y of up to kBandMaxN nodes in shared memory.
@@ -125,6 +126,10 @@ constexpr int kNmMaxBeads = 1536;
 // exterior spring forces' exchange part times -vb_bar).
 void launch_exchange_adjoint(const Sys& s, int D, double vb_bar, cudaStream_t st);
 void launch_exchange_estimators(const Sys& s, cudaStream_t st);
+// Its blocks at most (two per SM) and the doubles of Sys::epart.
+constexpr int kEstimatorThreads = 256;
+constexpr int kEstimatorBlocks = 304;
+constexpr int kEstimatorDoubles = 2 * kEstimatorBlocks;
 
 // factorial.cu: the factorial exchange (sum over all N! permutations) on
 // beads 1 and P, for at most kFactMaxN particles.  launch_factorial_sums

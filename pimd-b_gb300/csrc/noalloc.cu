@@ -46,7 +46,8 @@ constexpr size_t kOffV = kOffEt + kTri;                  // V, Vb, Vh, Vbh, yf, 
 constexpr size_t kOffRow = kOffV + 6 * kVec;             // rowR, rowC
 constexpr size_t kOffScal = kOffRow + 2 * kNoAllocMaxN;  // 4 scalars
 constexpr size_t kOffFlags = kOffScal + 4;               // 16 ints (8 doubles)
-constexpr size_t kScratchDoubles = kOffFlags + 8;
+constexpr size_t kOffEpart = kOffFlags + 8;              // the estimators' partial sums
+constexpr size_t kScratchDoubles = kOffEpart + kEstimatorDoubles;
 
 // About 1.1 MB per GPU.
 static __device__ __align__(256) double g_exchange_scratch[kScratchDoubles];
@@ -169,6 +170,7 @@ extern "C" int pimdb_exchange_noalloc(const double* ring, int nbeads, int natoms
     s.rowR = base + kOffRow;
     s.rowC = s.rowR + kNoAllocMaxN;
     s.scal = base + kOffScal;
+    s.epart = base + kOffEpart;
     s.xflags = reinterpret_cast<int*>(base + kOffFlags);
     s.err = s.xflags + 8;
     const int n4 = 4 * natoms * ndim;
