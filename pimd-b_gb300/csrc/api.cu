@@ -35,6 +35,7 @@ struct pimdb_handle {
     double* d_red[2] = {nullptr, nullptr};
     double* d_stage = nullptr;
     double* d_part = nullptr;  // pair-tile partial sums (Newton's third law path)
+    double* d_obs = nullptr;   // the energy and observable terms (obs_work), from the first call on
     int* d_err = nullptr;
     long long step = 0;
     // coordinate generation: advanced by every call that can change x; the
@@ -358,7 +359,7 @@ static void free_handle(pimdb_handle* h) {
     double* bufs[] = {h->s.x,   h->s.p,   h->s.f,   h->s.fphys, h->s.fx,   h->s.E,        h->s.V,
                       h->s.Vb,  h->s.scal, h->s.Vh, h->s.Vbh,  h->s.yf,   h->s.yb,       h->s.Wf,
                       h->s.Wb,  h->s.Et, h->s.rowR, h->s.rowC, h->d_C,  h->d_T,    h->d_rot,      h->d_red[0],
-                      h->d_red[1], h->d_stage, h->d_part, h->s.Vp, h->s.epart};
+                      h->d_red[1], h->d_stage, h->d_part, h->s.Vp, h->s.epart, h->d_obs};
     for (double* b : bufs)
         if (b) cudaFree(b);
     if (h->d_err) cudaFree(h->d_err);
@@ -1260,24 +1261,65 @@ extern "C" int pimdb_exchange_dbeta(pimdb_handle* h, double* dbeta) {
     return PIMDB_OK;
 }
 
+// The exchange beside other kernels: begins on the side stream (the handle's
+// stream when profiling, which times every launch there) ...
+static cudaStream_t fork_exchange(pimdb_handle* h) {
+    if (!h->s.bosonic || h->profile) return h->stream;
+    cudaEventRecord(h->fork_ev, h->stream);
+    cudaStreamWaitEvent(h->side, h->fork_ev, 0);
+    return h->side;
+}
+// ... and what follows on the handle's stream waits for it.
+static void join_exchange(pimdb_handle* h, cudaStream_t xs) {
+    if (xs == h->stream) return;
+    cudaEventRecord(h->join_ev, xs);
+    cudaStreamWaitEvent(h->stream, h->join_ev, 0);
+}
+
+// The per-block terms (`per` doubles per bead and block of energy_blocks) and
+// the estimators' tile energies, kept from the first call on.
+static int obs_work(pimdb_handle* h, double** part, double** tiles) {
+    const Sys& s = h->s;
+    const size_t n = (size_t)s.P * energy_blocks(s) * 7;
+    if (!h->d_obs)
+        CUDA_TRY(h, cudaMalloc((void**)&h->d_obs, (n + (h->d_part ? energy_tile_doubles(s) : 0)) * sizeof(double)));
+    *part = h->d_obs;
+    *tiles = h->d_obs + n;
+    return PIMDB_OK;
+}
+// Kernels of an energy evaluation: the tiles, when there are pairs and room
+// for their partial sums, and the per-bead terms.
+static int tile_launches(const pimdb_handle* h) {
+    return h->d_part && h->s.int_kind != PIMDB_POT_FREE && h->s.cutoff != 0.0 ? 2 : 1;
+}
+// SMs the tiles leave to an exchange on another stream (as enqueue_forces).
+static void reserve_for_exchange(pimdb_handle* h, bool beside) {
+    h->s.reserve_sms =
+        beside && h->d_part ? (h->opt_reserved_sms >= 0 ? h->opt_reserved_sms : exchange_reserved_sms(h->s)) : 0;
+}
+
 extern "C" int pimdb_potential_energy(pimdb_handle* h, double* terms) {
     if (!h || !terms) return fail(h, PIMDB_ERR_ARG, "NULL argument");
     complete_pending(h);
     const Sys& s = h->s;
     const int nb = energy_blocks(s);
     const size_t n = (size_t)s.P * nb * 3;
-    double* part = nullptr;
-    CUDA_TRY(h, cudaMalloc((void**)&part, n * sizeof(double)));
-    launch(h, PIMDB_K_BEAD_FORCES, [&] { launch_energy_terms(s, h->D, part, h->stream); });
+    double *part = nullptr, *tiles = nullptr;
+    const int ws = obs_work(h, &part, &tiles);
+    if (ws != PIMDB_OK) return ws;
+    const cudaStream_t xs = fork_exchange(h);
+    reserve_for_exchange(h, xs != h->stream);
     if (s.bosonic) {
-        exchange_front(h, h->stream);
-        if (h->factorial) exchange_scalars(h, false, h->stream);
+        exchange_front(h, xs);
+        if (h->factorial) exchange_scalars(h, false, xs);
     }
+    launch(h, PIMDB_K_BEAD_FORCES, [&] { launch_energy_terms(s, h->D, part, tiles, h->d_part, h->stream); },
+           tile_launches(h));
+    join_exchange(h, xs);
     std::vector<double> hp(n);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(hp.data(), part, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(part);
     if (e != cudaSuccess) return fail(h, PIMDB_ERR_CUDA, cudaGetErrorString(e));
     const int st = check_err_word(h);
     if (st != PIMDB_OK) return st;
@@ -1298,20 +1340,24 @@ extern "C" int pimdb_compute_observables(pimdb_handle* h, pimdb_observables* out
     const int D = h->D, P = s.P, N = s.N;
     const int nb = energy_blocks(s);
     const size_t n = (size_t)P * nb * 7;
-    double* part = nullptr;
-    CUDA_TRY(h, cudaMalloc((void**)&part, n * sizeof(double)));
-    launch(h, PIMDB_K_BEAD_FORCES, [&] { launch_observable_terms(s, D, part, h->stream); });
+    double *part = nullptr, *tiles = nullptr;
+    const int ws = obs_work(h, &part, &tiles);
+    if (ws != PIMDB_OK) return ws;
+    const cudaStream_t xs = fork_exchange(h);
+    reserve_for_exchange(h, xs != h->stream);
     if (s.bosonic) {
-        exchange_front(h, h->stream);
-        exchange_scalars(h, false, h->stream);
+        exchange_front(h, xs);
+        exchange_scalars(h, false, xs);
     }
+    launch(h, PIMDB_K_BEAD_FORCES, [&] { launch_observable_terms(s, D, part, tiles, h->d_part, h->stream); },
+           tile_launches(h));
+    join_exchange(h, xs);
     std::vector<double> hp(n);
     double sc[4] = {0.0, 0.0, 0.0, 0.0};
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(hp.data(), part, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess && s.bosonic) e = cudaMemcpyAsync(sc, s.scal, sizeof sc, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(part);
     if (e != cudaSuccess) return fail(h, PIMDB_ERR_CUDA, cudaGetErrorString(e));
     const int st = check_err_word(h);
     if (st != PIMDB_OK) return st;

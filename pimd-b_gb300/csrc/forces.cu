@@ -342,6 +342,11 @@ __device__ __forceinline__ double min_image_wrapped(double d, double L, long lon
 __device__ __noinline__ double pair_scale_exact(int kind, double r2, double param, const double* tbl) {
     return pair_scale_d<true>(kind, r2, param, tbl);
 }
+// The same with the pair energy: one exponential each for the repulsion and
+// the damping serve both.
+__device__ __noinline__ double aziz_scale_value_exact(double r2, const double* tbl, double& v) {
+    return aziz_scale_value(r2, tbl, v);
+}
 
 // One tile task: bead b, tile pair w (it <= jt) of the bead's T(T+1)/2.
 // kMixed: entries beyond the Aziz damping radius (and every entry of the
@@ -356,10 +361,20 @@ __device__ __noinline__ double pair_scale_exact(int kind, double r2, double para
 // within 1e-6 L of the half-box edge or within 1e-5 of the cutoff (where the
 // image or the in/out decision must be the FP64 one) take the exact FP64
 // path, as every marked entry does without kDf.
-template <int D, bool kMixed, bool kDf>
+//
+// kObs (with neither kMixed nor kDf): the estimators' tile.  Everything in
+// FP64, and beside the gradients the tile's pair energy and its virial term
+// (each pair's gradient times the coordinate of its first particle, not
+// wrapped) into obs[0] and obs[1].  Without a cutoff every pair is an entry.
+// Bound: the FP64 pipe, about 50 operations for a pair inside the cutoff,
+// evaluated once.  The per-particle loop it replaces took each pair from both
+// sides, inside the cutoff or not, with CUDA's exp and sqrt: the observables
+// of N = 256, P = 64 (Aziz, cutoff L/2) took 1.47 ms a call with it, 0.26 ms
+// with the tiles.
+template <int D, bool kMixed, bool kDf, bool kObs = false>
 __device__ __forceinline__ void compact_tile(const Sys& s, double* __restrict__ part, int T, int b, int w,
                                              CompactSmem<D>& sm, double (*g)[D], int cap, const double* tbl,
-                                             const dfl::ExpTable* etbl, int lane) {
+                                             const dfl::ExpTable* etbl, int lane, double* __restrict__ obs = nullptr) {
     using dfl::df;
     auto gd = reinterpret_cast<float2 (*)[D]>(g);  // kDf: gradient entries as (hi, lo)
     int it = 0, rem = w;  // row it holds the T - it tile pairs (it, it..T-1)
@@ -408,7 +423,7 @@ __device__ __forceinline__ void compact_tile(const Sys& s, double* __restrict__ 
         }
     }
     // 1. FP32 screen
-    const double cut = s.cutoff;
+    const double cut = kObs && s.cutoff < 0.0 ? (double)INFINITY : s.cutoff;
     const float cut2f = (float)(cut * cut) * 1.0001f;
     const bool aziz = s.int_kind == POT_AZIZ;
     const float near2f = aziz ? (float)(Aziz::D * Aziz::rm * Aziz::D * Aziz::rm) * 1.0001f : -1.0f;
@@ -438,7 +453,8 @@ __device__ __forceinline__ void compact_tile(const Sys& s, double* __restrict__ 
             }
             r2 = fmaf(d, d, r2);
         }
-        const bool in = ivalid && jl < nj && (!diag || st < 16 || lane < 16) && r2 <= cut2f;
+        // (kObs: without a cutoff a NaN separation is an entry too)
+        const bool in = ivalid && jl < nj && (!diag || st < 16 || lane < 16) && (kObs ? !(r2 > cut2f) : r2 <= cut2f);
         mask |= (unsigned)in << jl;
         const bool exact = aziz && (edge || (kDf && r2 >= shell2f));
         nmask |= (unsigned)(in && (r2 < near2f || exact)) << jl;
@@ -476,7 +492,6 @@ __device__ __forceinline__ void compact_tile(const Sys& s, double* __restrict__ 
     __syncwarp();
     const long long half_bits = __double_as_longlong(0.5 * s.L);
     const double cut2 = cut * cut;
-    const long long cut2_bits = __double_as_longlong(cut2);
     auto separation = [&](int f, double* r) {
         const int e = sm.fe[f], il = (e >> 5) & 31, jl = e & 31;
         double r2 = 0.0;
@@ -538,6 +553,18 @@ __device__ __forceinline__ void compact_tile(const Sys& s, double* __restrict__ 
         aid[a] = ajd[a] = df{0.0f, 0.0f};
     }
     const unsigned lt = (1u << lane) - 1u;
+    double ev = 0.0, vir = 0.0;  // kObs: this lane's pair energies and virial terms
+    // kObs: one evaluated entry (its gradient scale 0 and energy 0 beyond the cutoff)
+    auto observe = [&](int f, double v, double sc, const double* r) {
+        ev += v;
+        if (!diag) return;  // elsewhere every first particle is i: x_i . sum_j below
+        const int e = sm.fe[f], il = (e >> 5) & 31, jl = e & 31;
+        const int fl = min(il, jl);
+        double dot = 0.0;
+#pragma unroll
+        for (int a = 0; a < D; ++a) dot += s.x[idx<D>(s, b, a, it * kTile + fl)] * r[a];
+        vir += (il < jl ? sc : -sc) * dot;
+    };
     for (int c0 = 0; c0 < total; c0 += cap) {
         const int cend = min(total, c0 + cap), cn = cend - c0;
         auto store = [&](int f, double sc, const double* r) {
@@ -595,17 +622,37 @@ __device__ __forceinline__ void compact_tile(const Sys& s, double* __restrict__ 
                 }
             }
         } else if (aziz) {
-            // two independent entries per lane and iteration; entries inside
-            // the damping radius are redone below
+            // kObs (FP64 Aziz forces take kDf).  Two independent entries per
+            // lane and iteration; entries inside the damping radius are
+            // redone below
             for (int k = lane; k < cn; k += 64) {
                 const bool two = k + 32 < cn;
                 const int f0 = c0 + k, f1 = two ? f0 + 32 : f0;
-                double r0[D], r1[D];
+                double r0[D], r1[D], v0, v1;
                 const double q0 = separation_far(f0, r0), q1 = separation_far(f1, r1);
-                const double sc0 = aziz_far_scale(q0, tbl), sc1 = aziz_far_scale(q1, tbl);
-                // r2 >= 0: the cutoff test compares bit patterns (integer unit)
-                store(f0, __double_as_longlong(q0) < cut2_bits ? sc0 : 0.0, r0);
-                if (two) store(f1, __double_as_longlong(q1) < cut2_bits ? sc1 : 0.0, r1);
+                double sc0 = aziz_far_scale_value(q0, tbl, v0), sc1 = aziz_far_scale_value(q1, tbl, v1);
+                if (q0 >= cut2) sc0 = v0 = 0.0;
+                if (q1 >= cut2) sc1 = v1 = 0.0;
+                store(f0, sc0, r0);
+                if (!(sm.fe[f0] >> 15)) observe(f0, v0, sc0, r0);
+                if (two) {
+                    store(f1, sc1, r1);
+                    if (!(sm.fe[f1] >> 15)) observe(f1, v1, sc1, r1);
+                }
+            }
+        } else if (kObs) {
+            for (int k = lane; k < cn; k += 32) {
+                double r[D];
+                const double r2 = separation(c0 + k, r);
+                double sc = s.int_a, v = 0.5 * s.int_a * r2;  // harmonic
+                if (s.int_kind == POT_DIPOLE) {  // D / r^3 and -3 D / r^5
+                    const double ri = rsqrt_any(r2), ri2 = ri * ri;
+                    v = s.int_a * (ri2 * ri);
+                    sc = -3.0 * v * ri2;
+                }
+                if (r2 >= cut2) sc = v = 0.0;
+                store(c0 + k, sc, r);
+                observe(c0 + k, v, sc, r);
             }
         } else {
             for (int k = lane; k < cn; k += 32) {
@@ -670,6 +717,13 @@ __device__ __forceinline__ void compact_tile(const Sys& s, double* __restrict__ 
                         }
                         double r[D];
                         const double r2 = separation(fn, r);
+                        if (kObs) {
+                            double v = 0.0;
+                            const double sc = !(r2 >= cut2) ? aziz_scale_value_exact(r2, tbl, v) : 0.0;
+                            store(fn, sc, r);
+                            observe(fn, v, sc, r);
+                            continue;
+                        }
                         store(fn, r2 < cut2 ? pair_scale_exact(s.int_kind, r2, s.int_a, tbl) : 0.0, r);
                     }
                     __syncwarp();
@@ -711,6 +765,18 @@ __device__ __forceinline__ void compact_tile(const Sys& s, double* __restrict__ 
         for (int a = 0; a < D; ++a) {
             ai[a] = f32_to_f64(aid[a].hi) + f32_to_f64(aid[a].lo);
             aj[a] = f32_to_f64(ajd[a].hi) + f32_to_f64(ajd[a].lo);
+        }
+    }
+    if (kObs) {
+        if (!diag && i < s.N) {
+#pragma unroll
+            for (int a = 0; a < D; ++a) vir -= s.x[idx<D>(s, b, a, i)] * ai[a];  // ai = -sum_j grad
+        }
+        ev = warp_sum(ev);
+        vir = warp_sum(vir);
+        if (lane == 0) {
+            obs[0] = ev;
+            obs[1] = vir;
         }
     }
     const size_t base_b = (size_t)b * T;
@@ -766,9 +832,12 @@ __device__ __forceinline__ void tile_of_task(int task, int P, int T, int& b, int
 // pair warps.  The scheduler may place every block of a small grid there on
 // a busy GPU, so the warp that finishes last first takes whatever tasks are
 // left: the forces never depend on where blocks run.
-template <int D, bool kMixed, bool kDf>
+// kObs: the estimators' tiles, their energy and virial into
+// obs[(b * npairs + w) * 2 ..].
+template <int D, bool kMixed, bool kDf, bool kObs>
 __global__ void __launch_bounds__(32 * kCompactWarps) k_pair_tiles_compact(Sys s, double* __restrict__ part, int T,
-                                                                          int npairs, int* ctr, int cap, int nsm) {
+                                                                          int npairs, int* ctr, int cap, int nsm,
+                                                                          double* __restrict__ obs) {
     extern __shared__ __align__(16) unsigned char csm_raw[];
     __shared__ double tbl[256];
     __shared__ dfl::ExpTable etbl;
@@ -800,7 +869,8 @@ __global__ void __launch_bounds__(32 * kCompactWarps) k_pair_tiles_compact(Sys s
             if (task >= ntask) break;
             int b, w;
             tile_of_task(task, s.P, T, b, w);
-            compact_tile<D, kMixed, kDf>(s, part, T, b, w, sm, g, cap, tbl, &etbl, lane);
+            compact_tile<D, kMixed, kDf, kObs>(s, part, T, b, w, sm, g, cap, tbl, &etbl, lane,
+                                               kObs ? obs + ((size_t)b * npairs + w) * 2 : nullptr);
             __syncwarp();
         }
     };
@@ -1210,6 +1280,52 @@ size_t pair_partial_doubles(const Sys& s, int D) {
     return (size_t)s.P * T * D * s.ld + 1;
 }
 
+// The compact tiles of one launch: every bead's tile pairs by persistent
+// warps.  `obs` (else null): the estimators' form, FP64 in either precision.
+template <int D>
+static void compact_launch(const Sys& s, int mixed, double* part, int T, double* obs, cudaStream_t st) {
+    const int np = T * (T + 1) / 2;
+    const int cap = s.pair_cap > 0 ? std::min(s.pair_cap, kCompactMaxCap) : kCompactDefaultCap;
+    const size_t smem = compact_warp_bytes<D>(cap) * kCompactWarps;
+    // occupancy per device and variant, measured again when the entry cap
+    // changes (the attribute is set on the current device)
+    struct Occ {
+        int resident, cap, sms;
+    };
+    static Occ occ[64][4] = {};
+    static std::mutex occ_mu;
+    // FP64 with the Aziz potential: the double-float far path
+    const bool dfp = !mixed && s.int_kind == POT_AZIZ;
+    auto kern = obs ? k_pair_tiles_compact<D, false, false, true>
+                    : (mixed ? k_pair_tiles_compact<D, true, false, false>
+                             : (dfp ? k_pair_tiles_compact<D, false, true, false>
+                                    : k_pair_tiles_compact<D, false, false, false>));
+    const int variant = obs ? 3 : (mixed ? 1 : (dfp ? 2 : 0));
+    int dev = 0;
+    cudaGetDevice(&dev);
+    Occ o{};
+    {
+        std::lock_guard<std::mutex> lock(occ_mu);
+        Occ& slot = occ[(dev >= 0 && dev < 64) ? dev : 0][variant];
+        if (slot.cap != cap || dev < 0 || dev >= 64) {
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(compact_warp_bytes<D>(kCompactMaxCap) * kCompactWarps));
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&slot.resident, kern, 32 * kCompactWarps, smem);
+            cudaDeviceGetAttribute(&slot.sms, cudaDevAttrMultiProcessorCount, dev);
+            if (slot.resident < 1) slot.resident = 1;
+            slot.cap = cap;
+        }
+        o = slot;
+    }
+    const int sms = o.sms;
+    const int ntask = s.P * np;
+    const int blocks = std::min((ntask + kCompactWarps - 1) / kCompactWarps, o.resident * sms);
+    int* ctr = reinterpret_cast<int*>(part + (pair_partial_doubles(s, D) - 1));
+    Sys sr = s;
+    if (sms <= 16) sr.reserve_sms = 0;
+    kern<<<blocks, 32 * kCompactWarps, smem, st>>>(sr, part, T, np, ctr, cap, sms, obs);
+}
+
 template <int D>
 static void tiles_launch(const Sys& s, int mixed, int write_phys, double* part, cudaEvent_t before_finish, int add_fx,
                          cudaStream_t st) {
@@ -1218,43 +1334,7 @@ static void tiles_launch(const Sys& s, int mixed, int write_phys, double* part, 
     if (pairs) {
         const int np = T * (T + 1) / 2;
         if (s.cutoff > 0.0) {
-            const int cap = s.pair_cap > 0 ? std::min(s.pair_cap, kCompactMaxCap) : kCompactDefaultCap;
-            const size_t smem = compact_warp_bytes<D>(cap) * kCompactWarps;
-            // occupancy per device and precision, measured again when the
-            // entry cap changes (the attribute is set on the current device)
-            struct Occ {
-                int resident, cap, sms;
-            };
-            static Occ occ[64][3] = {};
-            static std::mutex occ_mu;
-            // FP64 with the Aziz potential: the double-float far path
-            const bool dfp = !mixed && s.int_kind == POT_AZIZ;
-            auto kern = mixed ? k_pair_tiles_compact<D, true, false>
-                              : (dfp ? k_pair_tiles_compact<D, false, true> : k_pair_tiles_compact<D, false, false>);
-            const int variant = mixed ? 1 : (dfp ? 2 : 0);
-            int dev = 0;
-            cudaGetDevice(&dev);
-            Occ o{};
-            {
-                std::lock_guard<std::mutex> lock(occ_mu);
-                Occ& slot = occ[(dev >= 0 && dev < 64) ? dev : 0][variant];
-                if (slot.cap != cap || dev < 0 || dev >= 64) {
-                    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(compact_warp_bytes<D>(kCompactMaxCap) * kCompactWarps));
-                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&slot.resident, kern, 32 * kCompactWarps, smem);
-                    cudaDeviceGetAttribute(&slot.sms, cudaDevAttrMultiProcessorCount, dev);
-                    if (slot.resident < 1) slot.resident = 1;
-                    slot.cap = cap;
-                }
-                o = slot;
-            }
-            const int sms = o.sms;
-            const int ntask = s.P * np;
-            const int blocks = std::min((ntask + kCompactWarps - 1) / kCompactWarps, o.resident * sms);
-            int* ctr = reinterpret_cast<int*>(part + (pair_partial_doubles(s, D) - 1));
-            Sys sr = s;
-            if (sms <= 16) sr.reserve_sms = 0;
-            kern<<<blocks, 32 * kCompactWarps, smem, st>>>(sr, part, T, np, ctr, cap, sms);
+            compact_launch<D>(s, mixed, part, T, nullptr, st);
         } else {
             dim3 grid((np + 3) / 4, s.P);
             if (mixed) k_pair_tiles<D, float><<<grid, 128, 0, st>>>(s, part, T, np);
@@ -1349,8 +1429,11 @@ __device__ __forceinline__ double pair_energy_ij(const Sys& s, const double* xi,
 }
 
 // part[(b * gridDim.x + block) * 3 + {0 external, 1 pair, 2 spring}]
+// `tiles` (else null): the pair energies of the estimators' tiles, `np` tile
+// pairs per bead, added up here instead of the all-pairs loop.
 template <int D>
-__global__ void __launch_bounds__(kEnergyThreads) k_energy_terms(Sys s, double* __restrict__ part) {
+__global__ void __launch_bounds__(kEnergyThreads) k_energy_terms(Sys s, double* __restrict__ part,
+                                                                 const double* __restrict__ tiles, int np) {
     __shared__ double xs[D][kEnergyThreads];
     __shared__ double red[3 * 32];
     const int b = blockIdx.y;
@@ -1365,7 +1448,9 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energy_terms(Sys s, double* 
         if (s.P > 1 && (!s.bosonic || b < s.P - 1)) e[2] = link_energy<D>(s, b, (b + 1) % s.P, i);
     }
     const bool pairs = s.int_kind != POT_FREE && s.cutoff != 0.0;
-    if (pairs) {
+    if (tiles) {
+        for (int w = i; w < np; w += gridDim.x * kEnergyThreads) e[1] += tiles[((size_t)b * np + w) * 2];
+    } else if (pairs) {
         for (int j0 = blockIdx.x * kEnergyThreads; j0 < s.N; j0 += kEnergyThreads) {
             __syncthreads();
             const int jl = j0 + threadIdx.x;
@@ -1448,10 +1533,15 @@ __global__ void k_local_energy(Sys s, int n, const int* __restrict__ items, doub
 //                              only the first particle's coordinate enters)
 //   [6] |grad_i (V_ext + sum_j V(r_ij))|^2 (the GSF force term)
 // part[((b * gridDim.x + block) * kObsTerms + k]
+// `tiles` (else null): [4] and [5] from the estimators' tiles, `np` tile
+// pairs per bead, and the pair gradients of [6] from their T slots `slots`;
+// otherwise every pair from both its sides in FP64 here.
 constexpr int kObsTerms = 7;
 
 template <int D>
-__global__ void __launch_bounds__(kEnergyThreads) k_observable_terms(Sys s, double* __restrict__ part) {
+__global__ void __launch_bounds__(kEnergyThreads) k_observable_terms(Sys s, double* __restrict__ part,
+                                                                     const double* __restrict__ tiles, int np,
+                                                                     const double* __restrict__ slots, int T) {
     __shared__ double xs[D][kEnergyThreads];
     __shared__ double red[kObsTerms * 32];
     const int b = blockIdx.y;
@@ -1480,7 +1570,17 @@ __global__ void __launch_bounds__(kEnergyThreads) k_observable_terms(Sys s, doub
         }
     }
     const bool pairs = s.int_kind != POT_FREE && s.cutoff != 0.0;
-    if (pairs) {
+    if (tiles) {
+        for (int w = i; w < np; w += gridDim.x * kEnergyThreads) {
+            t[4] += tiles[((size_t)b * np + w) * 2];
+            t[5] += tiles[((size_t)b * np + w) * 2 + 1];
+        }
+        if (active) {
+            for (int q = 0; q < T; ++q)
+#pragma unroll
+                for (int a = 0; a < D; ++a) g[a] -= slots[(((size_t)b * T + q) * D + a) * s.ld + i];
+        }
+    } else if (pairs) {
         for (int j0 = 0; j0 < s.N; j0 += kEnergyThreads) {
             __syncthreads();
             const int jl = j0 + threadIdx.x;
@@ -1530,20 +1630,44 @@ __global__ void __launch_bounds__(kEnergyThreads) k_observable_terms(Sys s, doub
     }
 }
 
-void launch_observable_terms(const Sys& s, int D, double* part, cudaStream_t st) {
-    dim3 grid((s.N + kEnergyThreads - 1) / kEnergyThreads, s.P);
-    if (D == 1) k_observable_terms<1><<<grid, kEnergyThreads, 0, st>>>(s, part);
-    else if (D == 2) k_observable_terms<2><<<grid, kEnergyThreads, 0, st>>>(s, part);
-    else k_observable_terms<3><<<grid, kEnergyThreads, 0, st>>>(s, part);
-}
-
 int energy_blocks(const Sys& s) { return (s.N + kEnergyThreads - 1) / kEnergyThreads; }
 
-void launch_energy_terms(const Sys& s, int D, double* part, cudaStream_t st) {
+// The estimators' tiles in front of the per-bead terms, when there are pair
+// forces and the tiles' partial sums (`slots`); returns the tiles per edge.
+size_t energy_tile_doubles(const Sys& s) {
+    const size_t T = (s.N + kTile - 1) / kTile;
+    return (size_t)s.P * T * (T + 1);
+}
+template <int D>
+static int energy_tiles(const Sys& s, double* tiles, double* slots, cudaStream_t st) {
+    if (!slots || s.int_kind == POT_FREE || s.cutoff == 0.0) return 0;
+    const int T = (s.N + kTile - 1) / kTile;
+    compact_launch<D>(s, 0, slots, T, tiles, st);
+    return T;
+}
+
+template <int D>
+static void observable_launch(const Sys& s, double* part, double* tiles, double* slots, cudaStream_t st) {
+    const int T = energy_tiles<D>(s, tiles, slots, st);
     dim3 grid(energy_blocks(s), s.P);
-    if (D == 1) k_energy_terms<1><<<grid, kEnergyThreads, 0, st>>>(s, part);
-    else if (D == 2) k_energy_terms<2><<<grid, kEnergyThreads, 0, st>>>(s, part);
-    else k_energy_terms<3><<<grid, kEnergyThreads, 0, st>>>(s, part);
+    k_observable_terms<D><<<grid, kEnergyThreads, 0, st>>>(s, part, T ? tiles : nullptr, T * (T + 1) / 2, slots, T);
+}
+void launch_observable_terms(const Sys& s, int D, double* part, double* tiles, double* slots, cudaStream_t st) {
+    if (D == 1) observable_launch<1>(s, part, tiles, slots, st);
+    else if (D == 2) observable_launch<2>(s, part, tiles, slots, st);
+    else observable_launch<3>(s, part, tiles, slots, st);
+}
+
+template <int D>
+static void energy_launch(const Sys& s, double* part, double* tiles, double* slots, cudaStream_t st) {
+    const int T = energy_tiles<D>(s, tiles, slots, st);
+    dim3 grid(energy_blocks(s), s.P);
+    k_energy_terms<D><<<grid, kEnergyThreads, 0, st>>>(s, part, T ? tiles : nullptr, T * (T + 1) / 2);
+}
+void launch_energy_terms(const Sys& s, int D, double* part, double* tiles, double* slots, cudaStream_t st) {
+    if (D == 1) energy_launch<1>(s, part, tiles, slots, st);
+    else if (D == 2) energy_launch<2>(s, part, tiles, slots, st);
+    else energy_launch<3>(s, part, tiles, slots, st);
 }
 
 void launch_local_energy(const Sys& s, int D, int n, const int* items, double* out, cudaStream_t st) {

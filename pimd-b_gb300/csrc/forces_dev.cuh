@@ -207,6 +207,12 @@ __device__ __forceinline__ double rsqrt_newton(double r2) {
     return fma(y0, e * fma(e, 0.375, 0.5), y0);
 }
 
+// rsqrt_newton where r2's float image is normal, CUDA's rsqrt elsewhere.
+__device__ __forceinline__ double rsqrt_any(double r2) {
+    const unsigned hi = (unsigned)__double2hiint(r2);  // 2^-100 <= r2 < 2^100
+    return hi - ((1023u - 100u) << 20) < (200u << 20) ? rsqrt_newton(r2) : rsqrt(r2);
+}
+
 // grad V(r) = s(r) * r for the radial pair potentials.  `r2` is |r|^2.
 template <typename R>
 __device__ __forceinline__ R pair_scale(int kind, R r2, R param);
@@ -272,6 +278,45 @@ __device__ __forceinline__ double aziz_far_scale(double r2, const double* tbl) {
     const double ri4 = ri2 * ri2;
     const double pa = fma(fma(c10, ri2, c8), ri2, c6);
     return fma(ri4 * ri4, pa, -e * rinv);
+}
+// The same with the pair energy (aziz.cpp:18-54 with F = 1): v = eps [A
+// exp(-alpha r_s) - C6 ix^6 - C8 ix^8 - C10 ix^10].
+__device__ __forceinline__ double aziz_far_scale_value(double r2, const double* tbl, double& v) {
+    constexpr double rm2 = Aziz::rm * Aziz::rm, rm6 = rm2 * rm2 * rm2, rm8 = rm6 * rm2, rm10 = rm8 * rm2;
+    constexpr double e6 = Aziz::C6 * Aziz::eps * rm6, e8 = Aziz::C8 * Aziz::eps * rm8, e10 = Aziz::C10 * Aziz::eps * rm10;
+    constexpr double c6 = 6.0 * e6, c8 = 8.0 * e8, c10 = 10.0 * e10;
+    const double rinv = rsqrt_any(r2);
+    const double e = exp_tang256(fma(-(Aziz::alpha / Aziz::rm), r2 * rinv, kAzizLnK), tbl);
+    const double ri2 = rinv * rinv;
+    const double ri4 = ri2 * ri2;
+    // e = A alpha eps / r_m exp(-alpha r_s)
+    v = fma(-(ri4 * ri2), fma(fma(e10, ri2, e8), ri2, e6), e * (Aziz::rm / Aziz::alpha));
+    return fma(ri4 * ri4, fma(fma(c10, ri2, c8), ri2, c6), -e * rinv);
+}
+// The general form of pair_scale_d for the Aziz potential with the energy of
+// pair_value beside it, from one exponential each.
+__device__ __forceinline__ double aziz_scale_value(double r2, const double* tbl, double& v) {
+    const double rinv = rsqrt(r2);
+    const double rs = r2 * rinv * (1.0 / Aziz::rm);
+    const double rep = Aziz::A * exp_tang256(-Aziz::alpha * rs, tbl);
+    double g = -Aziz::alpha * rep, u = rep;
+    if (!(rs > 1.0E-7 && rs < 0.01)) {
+        const double ix = Aziz::rm * rinv;  // 1 / r_scaled
+        const double ix2 = ix * ix;
+        const double ix6 = ix2 * ix2 * ix2;
+        const double pa = fma(fma(10.0 * Aziz::C10, ix2, 8.0 * Aziz::C8), ix2, 6.0 * Aziz::C6);
+        const double pb = fma(fma(Aziz::C10, ix2, Aziz::C8), ix2, Aziz::C6);
+        double F = 1.0, slope = ix * pa;
+        if (rs < Aziz::D) {
+            const double t = Aziz::D * ix - 1.0;
+            F = exp_tang256(-t * t, tbl);
+            slope -= 2.0 * Aziz::D * ix2 * t * pb;
+        }
+        g = fma(F * ix6, slope, g);
+        u = fma(-F * ix6, pb, u);
+    }
+    v = Aziz::eps * u;
+    return (Aziz::eps / Aziz::rm) * g * rinv;
 }
 // r_s = |r| / r_m >= D, on r2 = |r|^2 (a compare of the bit patterns: r2 >= 0)
 __device__ __forceinline__ bool aziz_is_far(double r2) {

@@ -53,9 +53,12 @@ void launch_pair_cells_and_finish(const Sys& s, int D, int nc, int mixed, int wr
 // and the local energy of listed (bead, particle) items ([n][2] ints).
 int energy_blocks(const Sys& s);
 // Per-bead observable terms, part[(b * energy_blocks + blk) * 7 + term]
-// (see k_observable_terms).
-void launch_observable_terms(const Sys& s, int D, double* part, cudaStream_t st);
-void launch_energy_terms(const Sys& s, int D, double* part, cudaStream_t st);
+// (see k_observable_terms).  With `slots` (pair_partial_doubles doubles) the
+// pairs are evaluated once each on the pair tiles, whose energies go to
+// `tiles` (energy_tile_doubles doubles).
+size_t energy_tile_doubles(const Sys& s);
+void launch_observable_terms(const Sys& s, int D, double* part, double* tiles, double* slots, cudaStream_t st);
+void launch_energy_terms(const Sys& s, int D, double* part, double* tiles, double* slots, cudaStream_t st);
 void launch_local_energy(const Sys& s, int D, int n, const int* items, double* out, cudaStream_t st);
 
 // exchange.cu: Feldman-Hirshberg exchange on beads 1 and P.
