@@ -625,6 +625,94 @@ __device__ void batch_exchange_forces_f32(const Sys& s, float* sm) {
     }
 }
 
+// The fresh FP32 estimate of a replica's potentials, by the whole block, one
+// direction after the other and one row per thread: replicas are small, and
+// the mixed path's FP32 forces round the solution relative to the estimate,
+// so its own arithmetic stays.  (The one-system kernels' estimate,
+// exchange_dev.cuh, inlined here instead cost the whole step 12%.)
+__device__ __forceinline__ void lse_add(float& mx, float& sm, float t) {
+    if (t > mx) {
+        sm = sm * __expf(mx - t) + 1.0f;
+        mx = t;
+    } else {
+        sm += __expf(t - mx);
+    }
+}
+// FP32 log-sum-exp node recursion.  fwd: value(n) = -(LSE - log n)/beta;
+// bwd: terms carry -log(N - r') and value(r) = -LSE/beta.
+__device__ inline void blocked_estimate(const double* __restrict__ Eg, int nn, int N, float beta, bool fwd, float* val,
+                                 float* amx, float* asm_) {
+    const int tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    for (int n = tid; n < nn; n += bd) {
+        amx[n] = -CUDART_INF_F;
+        asm_[n] = 0.0f;
+    }
+    __syncthreads();
+    const int nb = (nn + 31) / 32;
+    for (int b = 0; b < nb; ++b) {
+        const int base = 32 * b;
+        if (warp == 0) {
+            const int n = base + lane;
+            float mx = n < nn ? amx[n] : -CUDART_INF_F, sm = n < nn ? asm_[n] : 0.0f;
+            float e[32];
+#pragma unroll
+            for (int t = 0; t < 32; ++t) e[t] = (n < nn && n >= 1 && t < lane) ? (float)Eg[tri(n - 1) + base + t] : 0.0f;
+            float v = 0.0f;
+#pragma unroll
+            for (int t = 0; t < 32; ++t) {
+                if (lane == t && n < nn && n >= 1)
+                    v = -(mx + __logf(sm) - (fwd ? __logf((float)n) : 0.0f)) / beta;
+                const float vt = __shfl_sync(0xffffffffu, v, t);
+                if (lane > t && n < nn) {
+                    const int u = base + t;
+                    lse_add(mx, sm, -beta * (e[t] + vt) - (fwd ? 0.0f : __logf((float)(N - u))));
+                }
+            }
+            if (n < nn) val[n] = v;
+        }
+        __syncthreads();
+        for (int m = base + 32 + tid; m < nn; m += bd) {
+            float t[32];
+            float lmx = -CUDART_INF_F;
+#pragma unroll
+            for (int q = 0; q < 32; ++q) {
+                const int u = base + q;
+                t[q] = -beta * ((float)Eg[tri(m - 1) + u] + val[u]) - (fwd ? 0.0f : __logf((float)(N - u)));
+                lmx = fmaxf(lmx, t[q]);
+            }
+            float ls = 0.0f;
+#pragma unroll
+            for (int q = 0; q < 32; ++q) ls += __expf(t[q] - lmx);
+            float mx = amx[m], sm = asm_[m];
+            if (lmx > mx) {
+                sm = sm * __expf(mx - lmx) + ls;
+                mx = lmx;
+            } else {
+                sm += ls * __expf(lmx - mx);
+            }
+            amx[m] = mx;
+            asm_[m] = sm;
+        }
+        __syncthreads();
+    }
+}
+// Pass 1: the FP32 estimate of one direction (0 forward, 1 backward) by the
+// whole block; `fsm` holds 3 (N+1) floats.
+__device__ inline void batch_estimate(const Sys& s, int dir, float* fsm) {
+    const int N = s.N;
+    float* val = fsm;
+    float* amx = fsm + (N + 1);
+    float* asm_ = fsm + 2 * (N + 1);
+    const float beta = (float)s.beta_ex;
+    if (dir == 0) {
+        blocked_estimate(s.E, N + 1, N, beta, true, val, amx, asm_);
+        for (int m = threadIdx.x; m <= N; m += blockDim.x) s.Vh[m] = (double)val[m];
+    } else {
+        // nodes r = 0..N-1 <-> l = N..1
+        blocked_estimate(s.Et, N, N, beta, false, val, amx, asm_);
+        for (int l = threadIdx.x; l <= N; l += blockDim.x) s.Vbh[l] = (l >= 1) ? (double)val[N - l] : 0.0;
+    }
+}
 // The Feldman-Hirshberg exchange of one replica by the whole block; adds the
 // exterior springs to f on beads 1 and P (which hold the physical forces).
 // R = float: weights and exterior forces on the FP32 pipe (above).
@@ -644,9 +732,9 @@ __device__ void batch_exchange(const Sys& s, unsigned char* work, const double* 
     __syncthreads();
     for (int attempt = 0; attempt < 2; ++attempt) {
         if (fresh) {
-            estimate_direction(s, 0, reinterpret_cast<float*>(work));
+            batch_estimate(s, 0, reinterpret_cast<float*>(work));
             __syncthreads();
-            estimate_direction(s, 1, reinterpret_cast<float*>(work));
+            batch_estimate(s, 1, reinterpret_cast<float*>(work));
             __syncthreads();
         }
         if (kMixed) {

@@ -71,9 +71,9 @@ __global__ void k_exch_energies(Sys s) {
 // its band measurement).  With the previous potentials as the estimate, each
 // block forms its own row's weights (exch_weight, FP64) from the energies it
 // just wrote.  When a fresh estimate is due, the block that finishes last
-// runs it (both directions in turn) and then forms every weight in
-// double-float on the FP32 pipe (weights_df_block; on one SM the FP64
-// exponentials would take a quarter of a millisecond).  Four blocks per SM
+// runs it (both directions side by side) and then forms every weight with
+// double-float exponentials on the FP32 pipe (weights_df_block_f64arg; on one
+// SM the FP64 exponentials would take a quarter of a millisecond).  Four blocks per SM
 // bound the registers (the rare estimate's arrays would otherwise set them
 // for every row).
 constexpr int kEnergyRowThreads = 256;
@@ -162,14 +162,12 @@ __global__ void __launch_bounds__(kEnergyRowThreads, 4) k_exch_energies_rows(Sys
         if (fresh) atomicAdd(&s.xflags[kExchFreshCount], 1);
     }
     if (!fresh) return;
-    estimate_direction(s, 0, reinterpret_cast<float*>(rsm));
-    __syncthreads();
-    estimate_direction(s, 1, reinterpret_cast<float*>(rsm));
+    estimate_both(s, reinterpret_cast<float*>(rsm));
     __syncthreads();
     __shared__ dfl::ExpTable etbl;
     fill_exp_table_df(etbl);
     __syncthreads();
-    int band = weights_df_block(s, etbl, reinterpret_cast<float*>(rsm));
+    int band = weights_df_block_f64arg(s, etbl, reinterpret_cast<float*>(rsm));
     band = __reduce_max_sync(0xffffffffu, band);
     if ((threadIdx.x & 31) == 0 && band > 0) atomicMax(&s.xflags[kExchBand], band);
 }
@@ -178,7 +176,7 @@ __global__ void __launch_bounds__(kEnergyRowThreads, 4) k_exch_energies_rows(Sys
 // also runs the phase-0 estimate and weights).
 static size_t energies_rows_smem(const Sys& s) {
     return std::max(sizeof(double) * ((size_t)s.N + 2 * (((size_t)s.N + 31) / 32) + 2),
-                    sizeof(float) * 4 * ((size_t)s.N + 1));
+                    sizeof(float) * 6 * ((size_t)s.N + 1));  // the estimate of both directions
 }
 // The kernel's static shared memory (exp_tang's table, the double-float
 // exponential table, the last-block flag) counts against the 48 KB that a
@@ -321,6 +319,119 @@ __global__ void __launch_bounds__(kWaveThreads) k_exch_estimate(Sys s, int phase
     estimate_direction(s, blockIdx.x, fsm);
 }
 
+// Pass 1 across SMs, from the flat energies' size: on two blocks it took
+// 10.4 ms at N = 4096 and 0.71 ms at N = 777 (here 0.63 and 0.12 ms; 5 us per
+// block of nodes).  The schedule is
+// k_exch_solve_grid's (below): 32-node blocks go round-robin to `nct` CTAs per
+// direction (all resident: cooperative launch); the owner of block j + 1 folds
+// block j into it first, from entries loaded while it waited, resolves and
+// publishes it (g of its nodes, a fence, a flag), and then folds block j into
+// its other rows.  The critical path per block is a flag, one 32 x 32 fold and
+// 32 dependent log-sums.  Waits give up after a bounded number of polls
+// (ERRB_TIMEOUT).  The estimate itself goes to Vh / Vbh.
+__global__ void __launch_bounds__(kGridSolveThreads) k_exch_estimate_grid(Sys s, int phase, float* gsol,
+                                                                         unsigned* gflags, int nct) {
+    if (phase == 0) {
+        const int fresh = ((volatile int*)s.xflags)[3];
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            s.xflags[7] = !fresh;
+            if (fresh) atomicAdd(&s.xflags[kExchFreshCount], 1);
+        }
+        if (!fresh) return;
+    } else if (((volatile int*)s.xflags)[6] == 0) {
+        return;
+    }
+    extern __shared__ float esm[];
+    __shared__ float gj[32];
+    __shared__ int abort_estimate;
+    const int dir = blockIdx.x / nct, c = blockIdx.x % nct;
+    const EstDir d(s, dir);
+    const int nn = d.nn, nb = (nn + 31) / 32, nbmax = (s.N + 1 + 31) / 32;
+    const int nown = (nb - c + nct - 1) / nct;  // blocks c, c + nct, ...
+    float* gout = gsol + (size_t)dir * (s.N + 1);
+    unsigned* flags = gflags + (size_t)dir * nbmax;
+    float* mx = esm;               // [nown][32]
+    float* sm = esm + nown * 32;   // [nown][32]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int i = tid >> 3, part = tid & 7;  // fold role: row of the block, 4 of its 32 columns
+    for (int e = tid; e < nown * 32; e += blockDim.x) {
+        mx[e] = -CUDART_INF_F;
+        sm[e] = 0.0f;
+    }
+    if (tid == 0) abort_estimate = 0;
+    __syncthreads();
+    unsigned ed[32], en[4];  // the block resolved next: its diagonal block (warp 0), its rows against the block before
+    auto prefetch = [&](int b) {
+        if (warp == 0) est_load_diagonal(d, 32 * b, lane, ed);
+        if (b >= 1 && 32 * b + i < nn) est_load_row(d, 32 * b + i, b - 1, part, en);
+    };
+    auto diag_publish = [&](int b) {  // warp 0 of the owner of block b
+        const int n = 32 * b + lane, o = (b / nct) * 32 + lane;
+        const float g = est_diagonal(d, 32 * b, lane, n < nn ? mx[o] : 0.0f, n < nn ? sm[o] : 1.0f, ed);
+        if (n < nn) {
+            gout[n] = g;
+            est_store(s, d, n, g);
+        }
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) atomicExch(&flags[b], 1u);
+    };
+#pragma unroll
+    for (int q = 0; q < 4; ++q) en[q] = 0u;
+    if (c == 0) {
+        prefetch(0);
+        if (warp == 0) diag_publish(0);
+    }
+    if (nb > 1 && 1 % nct == c) prefetch(1);
+    for (int j = 0; j + 1 < nb; ++j) {
+        if (j % nct != c && tid == 0) {  // the owner of block j has it already
+            unsigned it = 0;
+            while (((volatile unsigned*)flags)[j] == 0u) {
+                if (++it > (1u << 22)) {
+                    atomicOr(s.err, ERRB_TIMEOUT);
+                    abort_estimate = 1;
+                    break;
+                }
+                if (it > 64) __nanosleep(32);
+            }
+            __threadfence();
+        }
+        __syncthreads();
+        if (abort_estimate) break;
+        if (tid < 32) gj[tid] = ((volatile float*)gout)[32 * j + tid];  // j + 1 < nb: a full block
+        __syncthreads();
+        const int jn = j + 1;
+        if (jn % nct == c) {  // the critical path: the next block's rows, then that block
+            const bool valid = 32 * jn + i < nn;
+            const int o = (jn / nct) * 32 + i;
+            est_fold(d, en, gj, part, valid, mx + o, sm + o);
+            __syncthreads();
+            if (warp == 0) diag_publish(jn);
+        }
+        for (int r = jn + (c - jn % nct + nct) % nct; r < nb; r += nct) {
+            if (r == jn) continue;
+            const bool valid = 32 * r + i < nn;
+            const int o = (r / nct) * 32 + i;
+            unsigned e[4] = {0u, 0u, 0u, 0u};
+            if (valid) est_load_row(d, 32 * r + i, j, part, e);
+            est_fold(d, e, gj, part, valid, mx + o, sm + o);
+        }
+        // entries for the next block this CTA resolves, while others work
+        if (jn + 1 < nb && (jn + 1) % nct == c) prefetch(jn + 1);
+        __syncthreads();
+    }
+    // the CTA that finishes last clears the flags for the next launch
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        if (atomicAdd(&gflags[2 * nbmax], 1u) == gridDim.x - 1) {
+            for (int e = 0; e < 2 * nbmax; ++e) gflags[e] = 0u;
+            gflags[2 * nbmax] = 0u;
+            __threadfence();
+        }
+    }
+}
+
 // Pass 2: every FP64 exponential at once, one thread per packed entry
 // (grid-stride over rows; phase 1 runs only on a retry).
 // Also records the band of the weights (kExchBand: the largest p + 1 - u of
@@ -391,7 +502,7 @@ __global__ void __launch_bounds__(kWaveThreads) k_exch_solve(Sys s, int force_ex
         if (threadIdx.x == 0) s.xflags[2] = 0;  // retry pending: phase 1 finishes
         return;
     }
-    solve_finish(s, !force_exact, &etbl);
+    solve_finish(s, !force_exact && phase == 0 && ((volatile int*)s.xflags)[7], &etbl);
     if (threadIdx.x == 0) {
         s.xflags[6] = 0;
         s.xflags[kExchBand] = 0;  // the next evaluation's weights measure it anew
@@ -574,7 +685,7 @@ __device__ __noinline__ void band_standalone_tail(const Sys& s, int dir, double*
     __syncthreads();
     if (*last_band == 0) return;
     __threadfence();
-    solve_finish(s, 1, &etbl);
+    solve_finish(s, *last_band != 3 && !allow_exact, &etbl);
     if (tid == 0) {
         s.xflags[6] = 0;
         // full exterior-force rows after a dense solve or a redone direction
@@ -699,7 +810,7 @@ __global__ void __launch_bounds__(kBandThreads) k_exch_solve_band(Sys s, int pha
     if (last_band == 0) return;
     __threadfence();
     if (last_band == 4) {
-        solve_finish(s, 1, &etbl);
+        solve_finish(s, ((volatile int*)s.xflags)[7], &etbl);
         if (tid == 0) {
             s.xflags[kExchBandLast] = s.xflags[kExchBand];
             s.xflags[kExchBand] = 0;  // the next evaluation's weights measure it anew
@@ -785,7 +896,7 @@ static void exchange_carveouts() {
                        (const void*)k_exch_energies_rows<2>, (const void*)k_exch_energies_rows<3>, (const void*)k_link_prefix<1>,
                        (const void*)k_link_prefix<2>, (const void*)k_link_prefix<3>,
                        (const void*)k_exch_energies_flat<1>, (const void*)k_exch_energies_flat<2>,
-                       (const void*)k_exch_energies_flat<3>, (const void*)k_exch_estimate,
+                       (const void*)k_exch_energies_flat<3>, (const void*)k_exch_estimate, (const void*)k_exch_estimate_grid,
                        (const void*)k_exch_weights, (const void*)k_exch_solve, (const void*)k_exch_solve_grid,
                        (const void*)k_exch_forces<1>, (const void*)k_exch_forces<2>, (const void*)k_exch_forces<3>};
     for (const void* f : k)
@@ -843,37 +954,56 @@ int launch_exchange_energies(const Sys& s, int D, cudaStream_t st, double* work)
     return 0;
 }
 
-// y of both directions for the banded solve and the multi-SM solve;
-// publication flags for the latter.
+// y of both directions for the banded solve and the multi-SM solve (and g
+// for the multi-SM estimate before them); publication flags for the latter.
 size_t exchange_grid_doubles(const Sys& s) { return 2 * ((size_t)s.N + 1); }
 size_t exchange_grid_flags(const Sys& s) {
-    return s.N >= kGridSolveMinN ? 2 * (((size_t)s.N + 1 + 31) / 32) + 1 : 1;
+    return s.N >= kFlatEnergiesMinN ? 2 * (((size_t)s.N + 1 + 31) / 32) + 1 : 1;
 }
 
-// The cooperative solve if every CTA can be resident; false otherwise.
-static bool grid_solve(const Sys& s, int phase, double* ysol, unsigned* gflags, int banded, cudaStream_t st) {
-    const int nb = (s.N + 1 + 31) / 32;
-    const int nct = nb < kGridSolveCtas ? nb : kGridSolveCtas;
-    const size_t smem = sizeof(double) * (((size_t)(nb + nct - 1) / nct) * 32 + 32);
-    // resident CTAs of the whole GPU, per device (0 = not measured yet)
-    static std::atomic<int> per_dev[64];
+// CTAs of kGridSolveThreads that are resident on the whole GPU at once, for
+// kernel `which` (0 solve, 1 estimate) with up to 8 KB of dynamic shared
+// memory; measured once per device.
+static int grid_resident(int which) {
+    static std::atomic<int> per_dev[2][64];  // 0 = not measured yet
     int dev = 0;
     cudaGetDevice(&dev);
-    int per = (dev >= 0 && dev < 64) ? per_dev[dev].load(std::memory_order_relaxed) - 1 : -1;
+    const bool known = dev >= 0 && dev < 64;
+    int per = known ? per_dev[which][dev].load(std::memory_order_relaxed) - 1 : -1;
     if (per < 0) {
         int sms = 0, b = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_exch_solve_grid, kGridSolveThreads, 4096) != cudaSuccess)
-            b = 0;
+        const void* k = which ? (const void*)k_exch_estimate_grid : (const void*)k_exch_solve_grid;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, kGridSolveThreads, 8192) != cudaSuccess) b = 0;
         per = b * sms;
-        if (dev >= 0 && dev < 64) per_dev[dev].store(per + 1, std::memory_order_relaxed);
+        if (known) per_dev[which][dev].store(per + 1, std::memory_order_relaxed);
     }
-    if (2 * nct > per) return false;
+    return per;
+}
+// CTAs per direction of the multi-SM kernels and the 32-node blocks each owns at most.
+static int grid_ctas(const Sys& s) { return std::min((s.N + 1 + 31) / 32, kGridSolveCtas); }
+static size_t grid_owned(const Sys& s) { return (size_t)((s.N + 1 + 31) / 32 + grid_ctas(s) - 1) / grid_ctas(s); }
+
+// The cooperative solve if every CTA can be resident; false otherwise.
+static bool grid_solve(const Sys& s, int phase, double* ysol, unsigned* gflags, int banded, cudaStream_t st) {
+    const int nct = grid_ctas(s);
+    if (2 * nct > grid_resident(0)) return false;
     Sys sc = s;
     int ph = phase, n = nct, bd = banded;
     void* args[] = {&sc, &ph, &ysol, &gflags, &n, &bd};
-    return cudaLaunchCooperativeKernel((void*)k_exch_solve_grid, dim3(2 * nct), dim3(kGridSolveThreads), args, smem,
-                                      st) == cudaSuccess;
+    return cudaLaunchCooperativeKernel((void*)k_exch_solve_grid, dim3(2 * nct), dim3(kGridSolveThreads), args,
+                                      sizeof(double) * (grid_owned(s) * 32 + 32), st) == cudaSuccess;
+}
+// The cooperative estimate likewise.
+static bool grid_estimate(const Sys& s, int phase, double* ysol, unsigned* gflags, cudaStream_t st) {
+    const int nct = grid_ctas(s);
+    if (2 * nct > grid_resident(1)) return false;
+    Sys sc = s;
+    int ph = phase, n = nct;
+    float* g = reinterpret_cast<float*>(ysol);
+    void* args[] = {&sc, &ph, &g, &gflags, &n};
+    return cudaLaunchCooperativeKernel((void*)k_exch_estimate_grid, dim3(2 * nct), dim3(kGridSolveThreads), args,
+                                      sizeof(float) * 2 * grid_owned(s) * 32, st) == cudaSuccess;
 }
 
 // SMs the pair tiles leave free while this exchange runs beside them: its
@@ -905,7 +1035,9 @@ int launch_exchange_recursions(const Sys& s, int exact, cudaStream_t st, double*
     int n = 0;
     for (int phase = 0; phase < (inline_retry ? 1 : 2); ++phase) {
         if (!(phase == 0 && estimate_done)) {  // else the energy kernel ran it
-            k_exch_estimate<<<2, kWaveThreads, esmem, st>>>(s, phase);
+            // across SMs from the flat energies' size, else on two blocks
+            if (!(s.N >= kFlatEnergiesMinN && ysol && gflags && grid_estimate(s, phase, ysol, gflags, st)))
+                k_exch_estimate<<<2, kWaveThreads, esmem, st>>>(s, phase);
             ++n;
         }
         if (!(phase == 0 && estimate_done)) {  // else the energy kernel formed them

@@ -8,6 +8,7 @@
 
 #include "common.cuh"
 #include "forces_dev.cuh"  // exp_tang
+#include "kernels.h"       // the exchange's flag indices
 
 namespace pimdb {
 __device__ __forceinline__ size_t tri(int v) { return (size_t)v * (size_t)(v + 1) / 2; }
@@ -75,82 +76,209 @@ __device__ inline void energy_row(const Sys& s, int v, int lane, const double* l
     }
     if (lane == 0 && v >= 1) s.Et[tri(s.N - v - 1) + (s.N - 1 - v)] = row[v];
 }
-__device__ __forceinline__ void lse_add(float& mx, float& sm, float t) {
-    if (t > mx) {
-        sm = sm * __expf(mx - t) + 1.0f;
-        mx = t;
-    } else {
-        sm += __expf(t - mx);
-    }
-}
 // The recursions as "node" recursions.  Forward: node n = level m = n,
 // node 0 known (V = 0), node n depends on nodes u < n through the packed row
 // E[n-1][u].  Backward: node r = N - l, node 0 (l = N) known, node r depends
 // on nodes r' < r through Et[r-1][r'] = E[p][l] with p = N - 1 - r' (so
 // p + 1 = N - r').  Both are evaluated by the same blocked scheme: nodes are
-// taken 32 at a time; warp 0 resolves the 32 nodes of a block one after the
-// other with shuffles (no barrier), then every thread folds the finished
-// block into the accumulators of all later nodes (one barrier pair per 32
-// nodes instead of one barrier per node).
+// taken 32 at a time; one warp resolves the 32 nodes of a block one after the
+// other with shuffles (no barrier), and the finished block is folded into the
+// accumulators of all later nodes.
 constexpr int kWaveThreads = 256;
-// FP32 log-sum-exp node recursion.  fwd: value(n) = -(LSE - log n)/beta;
-// bwd: terms carry -log(N - r') and value(r) = -LSE/beta.
-__device__ inline void blocked_estimate(const double* __restrict__ Eg, int nn, int N, float beta, bool fwd, float* val,
-                                 float* amx, float* asm_) {
-    const int tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, warp = tid >> 5;
-    for (int n = tid; n < nn; n += bd) {
-        amx[n] = -CUDART_INF_F;
-        asm_[n] = 0.0f;
+
+// ---- FP32 estimate.  In base-2 logarithms, with b = beta log2(e): node n's
+// log-sum is L_n = log2 sum_{u<n} 2^(g_u - b E[n-1][u]), and what it
+// contributes to later nodes is g_n = L_n - log2(n) forward (g_0 = 0),
+// g_n = L_n - log2(N - n) backward (g_0 = -log2(N)).  Forward V_n = -g_n / b,
+// backward value -L_n / b.  A running log-sum is a pair (mx, sm): 2^mx sm.
+__device__ __forceinline__ float ex2f(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float lg2f(float x) {
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// E for the estimate, from the double's upper word alone: sign, exponent and
+// 20 fraction bits (2^-20 relative is far below what the estimate needs; half
+// the bytes, no FP64-pipe conversion), 0 and 2^127 beyond a float's range.
+// est_load is volatile so that a thread's loads are all issued where they
+// stand instead of one by one in front of their uses (one L2 round trip per
+// block of nodes, not 32).
+__device__ __forceinline__ unsigned est_load(const double* p) {
+    unsigned v;
+    asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(reinterpret_cast<const unsigned*>(p) + 1));
+    return v;
+}
+__device__ __forceinline__ float est_value(unsigned hi) {
+    const unsigned e = (hi >> 20) & 0x7ffu;
+    if (e < 1023u - 126u) return 0.0f;
+    const unsigned q = e > 1023u + 126u ? 254u << 23 : (e - 896u) << 23 | (hi & 0xfffffu) << 3;
+    return __uint_as_float(hi & 0x80000000u | q);
+}
+struct EstDir {
+    const double* E;  // packed rows (s.E forward, s.Et backward)
+    int nn, N;
+    float b;  // beta log2(e)
+    bool fwd;
+    __device__ EstDir(const Sys& s, int dir)
+        : E(dir == 0 ? s.E : s.Et), nn(dir == 0 ? s.N + 1 : s.N), N(s.N),
+          b((float)(s.beta_ex * 1.4426950408889634)), fwd(dir == 0) {}
+    __device__ float norm(int n) const { return lg2f((float)(fwd ? n : N - n)); }
+};
+// One warp resolves the 32 nodes base .. base + 31: the lane's node's log-sum
+// over earlier blocks in (mx, sm), its row's entries of this block in e.
+// Returns g of the lane's node.
+__device__ __forceinline__ float est_diagonal(const EstDir& d, int base, int lane, float mx, float sm,
+                                              const unsigned (&e)[32]) {
+    const int n = base + lane;
+    const float nl = n >= 1 && n < d.nn ? d.norm(n) : 0.0f;
+    float g = 0.0f;
+#pragma unroll
+    for (int t = 0; t < 32; ++t) {
+        if (lane == t) g = n == 0 ? (d.fwd ? 0.0f : -d.norm(0)) : mx + lg2f(sm) - nl;
+        const float gt = __shfl_sync(0xffffffffu, g, t);
+        const float x = fmaf(-d.b, est_value(e[t]), gt), m = fmaxf(mx, x);
+        const float z = fmaf(sm, ex2f(mx - m), ex2f(x - m));
+        if (lane > t) {
+            sm = z;
+            mx = m;
+        }
     }
-    __syncthreads();
-    const int nb = (nn + 31) / 32;
-    for (int b = 0; b < nb; ++b) {
-        const int base = 32 * b;
-        if (warp == 0) {
-            const int n = base + lane;
-            float mx = n < nn ? amx[n] : -CUDART_INF_F, sm = n < nn ? asm_[n] : 0.0f;
-            float e[32];
+    return g;
+}
+// The lane's row entries of the diagonal block (0 where there are none).
+__device__ __forceinline__ void est_load_diagonal(const EstDir& d, int base, int lane, unsigned (&e)[32]) {
+    const int n = base + lane;
+    const bool row = n < d.nn && n >= 1;
+    const double* at = d.E + (row ? tri(n - 1) + base : 0);
 #pragma unroll
-            for (int t = 0; t < 32; ++t) e[t] = (n < nn && n >= 1 && t < lane) ? (float)Eg[tri(n - 1) + base + t] : 0.0f;
-            float v = 0.0f;
-#pragma unroll
-            for (int t = 0; t < 32; ++t) {
-                if (lane == t && n < nn && n >= 1)
-                    v = -(mx + __logf(sm) - (fwd ? __logf((float)n) : 0.0f)) / beta;
-                const float vt = __shfl_sync(0xffffffffu, v, t);
-                if (lane > t && n < nn) {
-                    const int u = base + t;
-                    lse_add(mx, sm, -beta * (e[t] + vt) - (fwd ? 0.0f : __logf((float)(N - u))));
-                }
-            }
-            if (n < nn) val[n] = v;
-        }
-        __syncthreads();
-        for (int m = base + 32 + tid; m < nn; m += bd) {
-            float t[32];
-            float lmx = -CUDART_INF_F;
-#pragma unroll
-            for (int q = 0; q < 32; ++q) {
-                const int u = base + q;
-                t[q] = -beta * ((float)Eg[tri(m - 1) + u] + val[u]) - (fwd ? 0.0f : __logf((float)(N - u)));
-                lmx = fmaxf(lmx, t[q]);
-            }
-            float ls = 0.0f;
-#pragma unroll
-            for (int q = 0; q < 32; ++q) ls += __expf(t[q] - lmx);
-            float mx = amx[m], sm = asm_[m];
-            if (lmx > mx) {
-                sm = sm * __expf(mx - lmx) + ls;
-                mx = lmx;
-            } else {
-                sm += ls * __expf(lmx - mx);
-            }
-            amx[m] = mx;
-            asm_[m] = sm;
-        }
-        __syncthreads();
+    for (int t = 0; t < 32; ++t) {
+        e[t] = 0u;
+        if (row && t < lane) e[t] = est_load(at + t);
     }
 }
+// Entries of row m against the 32 nodes of block j, four per thread of the
+// row's eight (columns part, part + 8, ...).
+__device__ __forceinline__ void est_load_row(const EstDir& d, int m, int j, int part, unsigned (&e)[4]) {
+    const double* row = d.E + tri(m - 1) + 32 * j + part;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) e[q] = est_load(row + 8 * q);
+}
+// Folds block j's nodes (gj[0..31]) into row m's log-sum; the eight threads
+// of a row call it together (`valid` false: only to take part).
+__device__ __forceinline__ void est_fold(const EstDir& d, const unsigned (&e)[4], const float* gj, int part, bool valid,
+                                         float* mx, float* sm) {
+    float t[4], m = -CUDART_INF_F;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        t[q] = fmaf(-d.b, est_value(e[q]), gj[part + 8 * q]);
+        m = fmaxf(m, t[q]);
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    float z = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) z += ex2f(t[q] - m);
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+    if (part == 0 && valid) {
+        const float a = *mx, n = fmaxf(a, m);
+        *sm = fmaf(*sm, ex2f(a - n), z * ex2f(m - n));
+        *mx = n;
+    }
+}
+// The estimate of node n into s.Vh / s.Vbh.
+__device__ __forceinline__ void est_store(const Sys& s, const EstDir& d, int n, float g) {
+    if (d.fwd) s.Vh[n] = (double)(-g / d.b);
+    else s.Vbh[d.N - n] = (double)(n == 0 ? 0.0f : -(g + d.norm(n)) / d.b);
+    if (!d.fwd && n == 0) s.Vbh[0] = 0.0;
+}
+
+// Pass 1 of one direction (0 forward, 1 backward) by `nt` threads (whole
+// warps, thread `t` of them; barrier `bar`, 0 for a whole block); `fsm` holds 3 (N + 1) floats.
+// Warp 0 resolves block b + 1 while the other warps fold block b into the
+// rows after it.  Both directions of N = 256 by one block of 256 threads, half
+// each: 72 us (one after the other with one thread per row, loads one by one:
+// about 300 us).  Out of line: a rare path whose arrays would otherwise set
+// the callers' registers.
+static __device__ __noinline__ void estimate_group(const Sys& s, int dir, float* fsm, int t, int nt, int bar) {
+    const EstDir d(s, dir);
+    const int nn = d.nn, lane = t & 31, warp = t >> 5;
+    float* g = fsm;
+    float* mx = fsm + (s.N + 1);
+    float* sm = fsm + 2 * (s.N + 1);
+    // barriers by constant ids: a block is charged for the ids it may use
+    auto sync = [&] {
+        if (bar == 0) __syncthreads();
+        else if (bar == 1) asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
+        else asm volatile("bar.sync 2, %0;" ::"r"(nt) : "memory");
+    };
+    for (int n = t; n < nn; n += nt) {
+        mx[n] = -CUDART_INF_F;
+        sm[n] = 0.0f;
+    }
+    sync();
+    // warp 0: the diagonal block's entries loaded ahead of their turn
+    unsigned e[32];
+    auto diagonal = [&](int b) {
+        const int n = 32 * b + lane;
+        const float v = est_diagonal(d, 32 * b, lane, n < nn ? mx[n] : 0.0f, n < nn ? sm[n] : 1.0f, e);
+        if (n < nn) {
+            g[n] = v;
+            est_store(s, d, n, v);
+        }
+    };
+    // rows lo .. hi - 1 against block j, by the threads t0 .. nt - 1; each
+    // warp takes eight rows at a time, every load issued before the first fold
+    auto fold = [&](int lo, int hi, int j, int t0) {
+        const int part = t & 7;
+        for (int m0 = lo + ((t - t0) >> 5) * 8 + (lane >> 3); m0 - (lane >> 3) < hi; m0 += ((nt - t0) >> 5) * 8) {
+            unsigned ea[4] = {0u, 0u, 0u, 0u}, eb[4] = {0u, 0u, 0u, 0u};
+            const bool va = m0 < hi, vb = m0 + 4 < hi;
+            if (va) est_load_row(d, m0, j, part, ea);
+            if (vb) est_load_row(d, m0 + 4, j, part, eb);
+            est_fold(d, ea, g + 32 * j, part, va, mx + m0, sm + m0);
+            est_fold(d, eb, g + 32 * j, part, vb, mx + m0 + 4, sm + m0 + 4);
+        }
+    };
+    const int nb = (nn + 31) / 32;
+    if (warp == 0) {
+        est_load_diagonal(d, 0, lane, e);
+        diagonal(0);
+    }
+    sync();
+    for (int b = 0; b + 1 < nb; ++b) {
+        const int next = 32 * (b + 1), after = min(nn, next + 32);
+        if (warp == 0) est_load_diagonal(d, next, lane, e);
+        fold(next, after, b, 0);
+        sync();
+        if (warp == 0) diagonal(b + 1);
+        if (nt == 32) fold(after, nn, b, 0);
+        else if (warp > 0) fold(after, nn, b, 32);
+        sync();
+    }
+}
+// One direction by the whole block; `fsm` holds 3 (N + 1) floats.
+__device__ inline void estimate_direction(const Sys& s, int dir, float* fsm) {
+    estimate_group(s, dir, fsm, threadIdx.x, blockDim.x, 0);
+}
+// Both directions by the whole block, side by side on half its warps each;
+// `fsm` holds 6 (N + 1) floats.
+__device__ inline void estimate_both(const Sys& s, float* fsm) {
+    const int nw = blockDim.x >> 5, h = nw / 2 * 32;
+    if (nw < 2) {
+        estimate_direction(s, 0, fsm);
+        estimate_direction(s, 1, fsm);
+    } else if ((int)threadIdx.x < h) {
+        estimate_group(s, 0, fsm, threadIdx.x, h, 1);
+    } else {
+        estimate_group(s, 1, fsm + 3 * (s.N + 1), threadIdx.x - h, blockDim.x - h, 2);
+    }
+}
+
 // FP64 triangular node solve: y(0) = 1, y(n) = sum_{u<n} W[n-1][u] y(u).
 __device__ inline void blocked_solve(const double* __restrict__ W, int nn, double* y, double* acc) {
     const int tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, warp = tid >> 5;
@@ -181,23 +309,6 @@ __device__ inline void blocked_solve(const double* __restrict__ W, int nn, doubl
             acc[m] = sacc;
         }
         __syncthreads();
-    }
-}
-// Pass 1: the FP32 estimate of one direction (0 forward, 1 backward) by the
-// whole block; `fsm` holds 3 (N+1) floats.
-__device__ inline void estimate_direction(const Sys& s, int dir, float* fsm) {
-    const int N = s.N;
-    float* val = fsm;
-    float* amx = fsm + (N + 1);
-    float* asm_ = fsm + 2 * (N + 1);
-    const float beta = (float)s.beta_ex;
-    if (dir == 0) {
-        blocked_estimate(s.E, N + 1, N, beta, true, val, amx, asm_);
-        for (int m = threadIdx.x; m <= N; m += blockDim.x) s.Vh[m] = (double)val[m];
-    } else {
-        // nodes r = 0..N-1 <-> l = N..1
-        blocked_estimate(s.Et, N, N, beta, false, val, amx, asm_);
-        for (int l = threadIdx.x; l <= N; l += blockDim.x) s.Vbh[l] = (l >= 1) ? (double)val[N - l] : 0.0;
     }
 }
 // Pass 2: the FP64 weights of packed entry (row p, column u), both directions
@@ -259,6 +370,60 @@ __device__ inline void weights_direction(const Sys& s, int dir, const double* tb
 // fresh estimate or the exact recursion), below -88 zero (a weight under
 // 1e-38 of the ones that normalise the row).  `vsm` holds 4 (N + 1) floats.
 // Returns this thread's band: the largest p + 1 - u of a nonzero weight.
+// weights_df_block_f64arg forms the argument in FP64 (only the exponential
+// in double-float): E, Vh_u and Vh_{p+1} are up to beta_ex V_B ~ 10^3-10^4 kT
+// and nearly cancel, so 48 bits of each leave 1e-11 in the weight.  Entries
+// whose FP32 argument is below -89 are zero without any FP64 operation.
+__device__ inline int weights_df_block_f64arg(const Sys& s, const dfl::ExpTable& etbl, float* vsm) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int N = s.N;
+    double* vh = reinterpret_cast<double*>(vsm);
+    double* vbh = vh + N + 1;
+    for (int m = threadIdx.x; m <= N; m += blockDim.x) {
+        vh[m] = s.Vh[m];
+        vbh[m] = s.Vbh[m];
+    }
+    __syncthreads();
+    const double nbeta = -s.beta_ex;
+    const float nbf = round_f32(nbeta);
+    int band = 0;
+    for (int p = warp; p < N; p += nw) {
+        const dfl::df inv = split_df(recip_row(p));
+        const double vp = vh[p + 1], vbp = vbh[p + 1];
+        const float vpf = round_f32(vp), vbpf = round_f32(vbp);
+        const size_t r = tri(p);
+        auto weight = [&](double E, double a, double b, float quick) {
+            if (quick < -89.0f) return 0.0;
+            const double x = nbeta * (E + a - b);
+            return df_to_f64(dfl::mul(dfl::exp(split_df(x), etbl), inv));
+        };
+        // four 32-entry chunks at a time, their loads issued together (the
+        // rows were just written by other SMs: an L2 round trip per group)
+        for (int u0 = lane; u0 <= p; u0 += 128) {
+            double E[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) E[k] = u0 + 32 * k <= p ? __ldcg(s.E + r + u0 + 32 * k) : 0.0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int u = u0 + 32 * k;
+                if (u > p) break;
+                const double vu = vh[u];
+                const float Ef = round_f32(E[k]);
+                const double wf = weight(E[k], vu, vp, nbf * (Ef + (round_f32(vu) - vpf)));
+                s.Wf[r + u] = wf;
+                bool nz = !f64_is_zero(wf);
+                if (u >= 1) {
+                    const double vbu = vbh[u];
+                    const double wb = weight(E[k], vbp, vbu, nbf * (Ef + (vbpf - round_f32(vbu))));
+                    s.Wb[tri(N - u - 1) + (N - 1 - p)] = wb;
+                    nz = nz || !f64_is_zero(wb);
+                }
+                if (nz) band = max(band, p + 1 - u);
+            }
+        }
+    }
+    return band;
+}
 __device__ inline int weights_df_block(const Sys& s, const dfl::ExpTable& etbl, float* vsm) {
     using dfl::df;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -394,7 +559,7 @@ __device__ inline int solve_direction(const Sys& s, int dir, int force_exact, do
         stale = __syncthreads_or(stale);
         if (tid == 0) {
             s.xflags[0] = bad;
-            s.xflags[4] = stale | nonfinite;
+            s.xflags[4] = (stale ? 1 : 0) | (nonfinite ? 2 : 0);
             if (nonfinite) atomicOr(s.err, ERRB_NONFINITE_VB);
         }
     } else {
@@ -436,7 +601,7 @@ __device__ inline int solve_direction(const Sys& s, int dir, int force_exact, do
         stale = __syncthreads_or(stale);
         if (tid == 0) {
             s.xflags[1] = bad;
-            s.xflags[5] = stale | nonfinite;
+            s.xflags[5] = (stale ? 1 : 0) | (nonfinite ? 2 : 0);
             if (nonfinite) atomicOr(s.err, ERRB_NONFINITE_VB);
         }
     }
@@ -446,8 +611,13 @@ __device__ inline int solve_direction(const Sys& s, int dir, int force_exact, do
 // probabilities, which need both V and V_backwards, and the estimates of the
 // next evaluation: V, V_backwards themselves or, with `extrapolate` and a
 // previous result in s.Vp (NaN until there is one), the linear extrapolation
-// 2 V(t) - V(t - dt), which smooth dynamics keep much closer.  With `et` the
-// row exponentials in double-float (exp_df).
+// 2 V(t) - V(t - dt), which smooth dynamics keep much closer.  The caller
+// asks for no extrapolation after an evaluation from a fresh estimate: the
+// coordinates may have jumped, and 2 V - V(before the jump) would fail again
+// (one more fresh estimate, 10 ms at N = 4096).  An estimate that was not
+// extrapolated and is 30 kT off asks for no fresh one either: the next, which
+// is, will be far closer.  With `et` the row exponentials in double-float
+// (exp_df).
 __device__ inline void solve_finish(const Sys& s, int extrapolate = 0, const dfl::ExpTable* et = nullptr) {
     const int N = s.N, tid = threadIdx.x, bd = blockDim.x;
     const double beta = s.beta_ex;
@@ -461,7 +631,9 @@ __device__ inline void solve_finish(const Sys& s, int extrapolate = 0, const dfl
         s.rowC[l] = et ? exp_df(aC, *et) : exp(aC);
     }
     __syncthreads();
-    const int need = ((volatile int*)s.xflags)[4] | ((volatile int*)s.xflags)[5];
+    // [4], [5] per direction: 1 the estimate was 30 kT off, 2 not finite
+    const int off = ((volatile int*)s.xflags)[4] | ((volatile int*)s.xflags)[5];
+    const int need = (off & 2) || ((off & 1) && (!s.Vp || ((volatile int*)s.xflags)[kExchOrder]));
     for (int m = tid; m <= N; m += bd) {
         const double v = V[m], vb = m >= 1 ? Vb[m] : 0.0;
         if (s.Vp && extrapolate && isfinite(s.Vp[m]) && isfinite(s.Vp[N + 1 + m])) {
@@ -476,9 +648,11 @@ __device__ inline void solve_finish(const Sys& s, int extrapolate = 0, const dfl
             s.Vp[N + 1 + m] = vb;
         }
     }
+    __syncthreads();  // every thread has read the flags
     if (tid == 0) {
         s.xflags[2] = 0;
         s.xflags[3] = need;
+        if (s.Vp) s.xflags[kExchOrder] = extrapolate;
         s.Vb[0] = VN;  // V_backwards[0] = V[N] (:127)
         s.scal[0] = VN;
     }

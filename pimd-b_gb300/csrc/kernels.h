@@ -104,6 +104,9 @@ constexpr int kExchBandDone = 14;
 // completed (0 when another path solved it): the exterior-force rows skip
 // the entries beyond it, all exact zeros.
 constexpr int kExchBandLast = 15;
+// Index in Sys::xflags (with Sys::Vp only) of whether the estimate waiting in
+// Vh is extrapolated from the last two results (else it is the last one).
+constexpr int kExchOrder = 8;
 // Index in Sys::xflags of the count of finished blocks of the per-row energy
 // kernel (its last block runs a due FP32 estimate) and of the estimators' (its
 // last block forms the scalars); 0 between launches.
