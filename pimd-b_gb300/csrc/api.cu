@@ -75,9 +75,7 @@ struct pimdb_handle {
     double* d_nh = nullptr;
     double* d_pnm = nullptr;
     int opt_cells = -1;
-    // factorial exchange (sum over all N! permutations): its work buffer
-    bool factorial = false;
-    double* d_fact = nullptr;
+    bool factorial = false;  // the exchange is the sum over all N! permutations
     // RanMars parity noise: the streams and the staged normals (Sys::noise)
     RanMarsState* d_rng = nullptr;
     double* d_noise = nullptr;
@@ -370,7 +368,6 @@ static void free_handle(pimdb_handle* h) {
     if (h->d_modes) cudaFree(h->d_modes);
     if (h->d_cells) cudaFree(h->d_cells);
     if (h->d_nh) cudaFree(h->d_nh);
-    if (h->d_fact) cudaFree(h->d_fact);
     if (h->d_rng) cudaFree(h->d_rng);
     if (h->h_err) cudaFreeHost(h->h_err);
     if (h->d_ysol) cudaFree(h->d_ysol);
@@ -463,8 +460,6 @@ extern "C" int pimdb_create(const pimdb_config* cfg, void* cuda_stream, pimdb_ha
     h->cell_nc = cell_grid(s, h->D);
     if (e == cudaSuccess && h->cell_nc > 0) e = cudaMalloc(&h->d_cells, cell_buffer_bytes(s, h->D, h->cell_nc));
     h->factorial = s.bosonic && c.exchange == PIMDB_EXCHANGE_FACTORIAL;
-    if (e == cudaSuccess && h->factorial)
-        e = cudaMalloc((void**)&h->d_fact, factorial_work_doubles(s.N) * sizeof(double));
     if (e == cudaSuccess && c.rng == PIMDB_RNG_RANMAR && c.thermostat == PIMDB_THERMO_LANGEVIN) {
         std::vector<RanMarsState> st((size_t)s.P);
         for (int b = 0; b < s.P; ++b) ranmars_seed((int)(c.seed + (unsigned long long)b), st[b]);
@@ -702,15 +697,12 @@ extern "C" int pimdb_get_step(pimdb_handle* h, long long* step) {
 
 // The exchange on beads 1 and P in two parts.  exchange_front: everything
 // up to the forces (Feldman-Hirshberg: cycle energies and the V / V_backwards
-// recursions, which give V_B; factorial: the permutation sums).
-// exchange_forces: the exterior spring forces into fx, also added into f
-// with `accumulate` (factorial: also every scalar).
+// recursions, which give V_B; factorial: nothing).  exchange_forces: the
+// exterior spring forces into fx, also added into f with `accumulate`
+// (factorial: the whole exchange).
 static void exchange_front(pimdb_handle* h, cudaStream_t st) {
     const Sys& s = h->s;
-    if (h->factorial) {
-        launch(h, PIMDB_K_EXCH_RECURSIONS, [&] { launch_factorial_sums(s, h->D, h->d_fact, st); }, 2);
-        return;
-    }
+    if (h->factorial) return;
     int est = 0;
     launch(h, PIMDB_K_EXCH_ENERGIES, [&] { est = launch_exchange_energies(s, h->D, st, h->d_ework); },
            h->d_ework ? 2 : 1);
@@ -723,7 +715,7 @@ static void exchange_front(pimdb_handle* h, cudaStream_t st) {
 static void exchange_forces(pimdb_handle* h, int accumulate, cudaStream_t st) {
     const Sys& s = h->s;
     if (h->factorial)
-        launch(h, PIMDB_K_EXCH_FORCES, [&] { launch_factorial_finish(s, h->D, h->d_fact, accumulate, st); });
+        launch(h, PIMDB_K_EXCH_FORCES, [&] { launch_factorial(s, h->D, accumulate, st); });
     else
         launch(h, PIMDB_K_EXCH_FORCES, [&] { launch_exchange_forces_mode(s, h->D, accumulate, st); });
 }

@@ -138,15 +138,11 @@ constexpr int kEstimatorBlocks = 304;
 constexpr int kEstimatorDoubles = 2 * kEstimatorBlocks;
 
 // factorial.cu: the factorial exchange (sum over all N! permutations) on
-// beads 1 and P, for at most kFactMaxN particles.  launch_factorial_sums
-// (2 kernels) fills `work` (factorial_work_doubles(N) doubles);
-// launch_factorial_finish then writes the scalars (V_B, primEstimator, 0, 0)
-// and the exterior spring forces into fx (and adds them into f with
-// `accumulate`).
+// beads 1 and P, for at most kFactMaxN particles, in one launch: the scalars
+// (V_B, primEstimator, 0, 0) and the exterior spring forces into fx (and
+// added into f with `accumulate`).
 constexpr int kFactMaxN = 12;
-size_t factorial_work_doubles(int N);
-int launch_factorial_sums(const Sys& s, int D, double* work, cudaStream_t st);
-void launch_factorial_finish(const Sys& s, int D, double* work, int accumulate, cudaStream_t st);
+void launch_factorial(const Sys& s, int D, int accumulate, cudaStream_t st);
 
 // RanMars parity noise (integrator.cu): one RanMars stream per bead,
 // seeded on the host (ranmars_seed: seed in 1..900000000), drawn on the
