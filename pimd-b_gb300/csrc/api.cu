@@ -771,7 +771,7 @@ static void enqueue_forces(pimdb_handle* h) {
                 launch_pair_tiles_and_finish(s, h->D, mixed, nm ? 1 : 0, h->d_part, before_finish, fx_in_finish,
                                              h->stream);
             },
-            pairs ? 2 : 1);
+            pair_tile_kernels(s, mixed));
     } else {
         launch(h, PIMDB_K_BEAD_FORCES, [&] { launch_bead_forces(s, h->D, mixed, nm ? 1 : 0, h->stream); });
     }

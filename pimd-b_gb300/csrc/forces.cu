@@ -894,6 +894,29 @@ __global__ void __launch_bounds__(32 * kCompactWarps) k_pair_tiles_compact(Sys s
     }
 }
 
+// One force component: springs + `acc`, the physical force (-grad V_ext and
+// the pair forces) of particle i of bead b along axis a, whose coordinate is xi.
+template <int D>
+__device__ __forceinline__ void finish_component(const Sys& s, int b, int a, int i, double xi, double acc,
+                                                 int write_phys, int add_fx) {
+    const size_t o = idx<D>(s, b, a, i);
+    if (write_phys) s.fphys[o] = acc;
+    if (s.bosonic && (b == 0 || b == s.P - 1)) {
+        // exterior springs from the exchange (fx, written beside the pair
+        // forces) or, without add_fx, added by the exchange force kernel
+        s.f[o] = add_fx ? acc + s.fx[((size_t)(b == 0 ? 0 : 1) * D + a) * s.ld + i] : acc;
+    } else {
+        const int bp = (b - 1 + s.P) % s.P, bn = (b + 1) % s.P;
+        double dp = s.x[idx<D>(s, bp, a, i)] - xi;
+        double dn = s.x[idx<D>(s, bn, a, i)] - xi;
+        if (s.pbc) {
+            dp = min_image(dp, s.L, s.invL);
+            dn = min_image(dn, s.L, s.invL);
+        }
+        s.f[o] = s.kappa * (dp + dn) + acc;
+    }
+}
+
 // f = springs + (-grad V_ext + sum of the pair slots), one thread per
 // (bead, axis, particle).  T = 0 when there are no pair forces.
 template <int D>
@@ -910,21 +933,48 @@ __global__ void k_bead_finish(Sys s, const double* __restrict__ part, int T, int
     ext_force<D>(s, xi, fe);
     double acc = fe[a];
     for (int q = 0; q < T; ++q) acc += part[(((size_t)b * T + q) * D + a) * s.ld + i];
-    const size_t o = idx<D>(s, b, a, i);
-    if (write_phys) s.fphys[o] = acc;
-    if (s.bosonic && (b == 0 || b == s.P - 1)) {
-        // exterior springs from the exchange (fx, written beside the pair
-        // forces) or, without add_fx, added by the exchange force kernel
-        s.f[o] = add_fx ? acc + s.fx[((size_t)(b == 0 ? 0 : 1) * D + a) * s.ld + i] : acc;
-    } else {
-        const int bp = (b - 1 + s.P) % s.P, bn = (b + 1) % s.P;
-        double dp = s.x[idx<D>(s, bp, a, i)] - xi[a];
-        double dn = s.x[idx<D>(s, bn, a, i)] - xi[a];
-        if (s.pbc) {
-            dp = min_image(dp, s.L, s.invL);
-            dn = min_image(dn, s.L, s.invL);
-        }
-        s.f[o] = s.kappa * (dp + dn) + acc;
+    finish_component<D>(s, b, a, i, xi[a], acc, write_phys, add_fx);
+}
+
+// The whole force evaluation with the harmonic interaction of every pair
+// (FP64; harmonic_all_pairs): one block per (bead, axis) row, its sum first.
+// N = 61, P = 20: 5 us in place of the pair tiles' 22 and k_bead_finish's 5.
+constexpr int kRowThreads = 128;
+template <int D>
+__global__ void __launch_bounds__(kRowThreads) k_bead_finish_harmonic(Sys s, int write_phys, int add_fx) {
+    __shared__ double sh[kRowThreads / 32], sl[kRowThreads / 32];
+    const int b = blockIdx.x / D, a = blockIdx.x - b * D;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double* row = s.x + idx<D>(s, b, a, 0);
+    const double ref = row[0];
+    double hi = 0.0, lo = 0.0;
+    for (int i = threadIdx.x; i < s.N; i += kRowThreads) add_to_pair(row[i] - ref, hi, lo);
+    warp_sum_pair(hi, lo);
+    if (lane == 0) {
+        sh[warp] = hi;
+        sl[warp] = lo;
+    }
+    __syncthreads();
+    hi = sh[0];
+    lo = sl[0];
+#pragma unroll
+    for (int w = 1; w < kRowThreads / 32; ++w) {
+        add_to_pair(sh[w], hi, lo);
+        lo += sl[w];
+    }
+    for (int i = threadIdx.x; i < s.N; i += kRowThreads) {
+        double xi[D], fe[D];
+#pragma unroll
+        for (int c = 0; c < D; ++c) xi[c] = s.x[idx<D>(s, b, c, i)];
+        ext_force<D>(s, xi, fe);
+        double x = xi[0], acc = fe[0];
+#pragma unroll
+        for (int c = 1; c < D; ++c)
+            if (a == c) {
+                x = xi[c];
+                acc = fe[c];
+            }
+        finish_component<D>(s, b, a, i, x, acc + harmonic_all_force(s, x - ref, hi, lo), write_phys, add_fx);
     }
 }
 
@@ -1280,6 +1330,14 @@ size_t pair_partial_doubles(const Sys& s, int D) {
     return (size_t)s.P * T * D * s.ld + 1;
 }
 
+// Kernels of launch_pair_tiles_and_finish: without pairs, or with the
+// harmonic interaction of every pair in FP64 (O(N), in the finishing kernel;
+// mixed precision keeps its FP32 pair arithmetic), only the finishing one.
+int pair_tile_kernels(const Sys& s, int mixed) {
+    if (s.int_kind == POT_FREE || s.cutoff == 0.0) return 1;
+    return !mixed && s.int_kind == POT_HARMONIC && s.cutoff < 0.0 && !s.pbc ? 1 : 2;
+}
+
 // The compact tiles of one launch: every bead's tile pairs by persistent
 // warps.  `obs` (else null): the estimators' form, FP64 in either precision.
 template <int D>
@@ -1331,6 +1389,11 @@ static void tiles_launch(const Sys& s, int mixed, int write_phys, double* part, 
                          cudaStream_t st) {
     const bool pairs = s.int_kind != POT_FREE && s.cutoff != 0.0;
     const int T = pairs ? (s.N + kTile - 1) / kTile : 0;
+    if (pair_tile_kernels(s, mixed) == 1 && pairs) {
+        if (before_finish) cudaStreamWaitEvent(st, before_finish, 0);
+        k_bead_finish_harmonic<D><<<s.P * D, kRowThreads, 0, st>>>(s, write_phys, add_fx);
+        return;
+    }
     if (pairs) {
         const int np = T * (T + 1) / 2;
         if (s.cutoff > 0.0) {

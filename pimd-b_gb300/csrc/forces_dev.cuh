@@ -381,6 +381,40 @@ __device__ __forceinline__ void ext_force(const Sys& s, const double* xi, double
     }
 }
 
+// The harmonic interaction of every pair without a cutoff or images, F_i =
+// -k sum_j (x_i - x_j), is linear: F_i = k (S - N y_i) with y = x - x_0 and
+// S = sum_j y_j, N operations a bead instead of N^2.  Taken relative to
+// particle 0, so that a cloud far from the origin loses nothing; S as an
+// unevaluated sum hi + lo (two_sum), so that it is as good as exact.
+__device__ __forceinline__ bool harmonic_all_pairs(const Sys& s) {
+    return s.int_kind == POT_HARMONIC && s.cutoff < 0.0 && !s.pbc;
+}
+__device__ __forceinline__ void two_sum_f64(double a, double b, double& h, double& l) {
+    h = a + b;
+    const double t = h - a;
+    l = (a - (h - t)) + (b - t);
+}
+// (hi, lo) += v
+__device__ __forceinline__ void add_to_pair(double v, double& hi, double& lo) {
+    double h, l;
+    two_sum_f64(hi, v, h, l);
+    hi = h;
+    lo += l;
+}
+__device__ __forceinline__ void warp_sum_pair(double& hi, double& lo) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double ph = __shfl_xor_sync(0xffffffffu, hi, o), pl = __shfl_xor_sync(0xffffffffu, lo, o);
+        double h, l;
+        two_sum_f64(hi, ph, h, l);
+        hi = h;
+        lo = (lo + pl) + l;
+    }
+}
+__device__ __forceinline__ double harmonic_all_force(const Sys& s, double y, double hi, double lo) {
+    return s.int_a * (fma(-(double)s.N, y, hi) + lo);
+}
+
 // Pair potential V(r) of one separation (`r2` = |r|^2), the reference's
 // V() for one distance vector: harmonic.cpp:7-19 (1/2 k r^2), dipole.cpp:5-20
 // (D / r^3), aziz.cpp:18-54 with F of aziz.h:25-27.
