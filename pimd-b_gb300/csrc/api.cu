@@ -83,7 +83,6 @@ struct pimdb_handle {
     // the exchange's triangular solve across SMs (large N): y of both
     // directions and the publication flags
     double* d_ysol = nullptr;
-    double* d_cm = nullptr;  // the pending COM correction, reduced (3 doubles)
     double* d_ework = nullptr;  // link prefix sums and wrapped end beads (large N)
     unsigned* d_gflags = nullptr;
     // CUDA graphs of pimdb_step_async: keyed by the step count and the
@@ -371,7 +370,6 @@ static void free_handle(pimdb_handle* h) {
     if (h->d_rng) cudaFree(h->d_rng);
     if (h->h_err) cudaFreeHost(h->h_err);
     if (h->d_ysol) cudaFree(h->d_ysol);
-    if (h->d_cm) cudaFree(h->d_cm);
     if (h->d_ework) cudaFree(h->d_ework);
     if (h->d_gflags) cudaFree(h->d_gflags);
     if (h->d_noise) cudaFree(h->d_noise);
@@ -444,7 +442,6 @@ extern "C" int pimdb_create(const pimdb_config* cfg, void* cuda_stream, pimdb_ha
         if (e == cudaSuccess) e = cudaMemset(s.Vp, 0xff, 2 * ((size_t)s.N + 1) * sizeof(double));
     }
     if (e == cudaSuccess && s.bosonic) e = alloc(&s.epart, kEstimatorDoubles);
-    if (e == cudaSuccess) e = alloc(&h->d_cm, 3);
     if (e == cudaSuccess && s.bosonic && exchange_energy_doubles(s, h->D) > 0)
         e = alloc(&h->d_ework, exchange_energy_doubles(s, h->D));
     if (e == cudaSuccess && s.bosonic && exchange_grid_doubles(s) > 0) {
@@ -479,8 +476,8 @@ extern "C" int pimdb_create(const pimdb_config* cfg, void* cuda_stream, pimdb_ha
     if (e == cudaSuccess) e = cudaMemset(s.xflags, 0, 16 * sizeof(int));
     const int one = 1;
     if (e == cudaSuccess) e = cudaMemcpy(s.xflags + 3, &one, sizeof(int), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = alloc(&h->d_red[0], (size_t)3 * nred);
-    if (e == cudaSuccess) e = alloc(&h->d_red[1], (size_t)3 * nred);
+    if (e == cudaSuccess) e = alloc(&h->d_red[0], com_doubles(nred));
+    if (e == cudaSuccess) e = alloc(&h->d_red[1], com_doubles(nred));
     // host-order staging for the state crossing the boundary: [3][P*N*D]
     if (e == cudaSuccess) e = alloc(&h->d_stage, (size_t)3 * s.P * s.N * h->D);
     if (e == cudaSuccess) e = cudaMallocHost((void**)&h->h_err, sizeof(int));
@@ -832,12 +829,12 @@ static void nose_hoover(pimdb_handle* h) {
     }, nmc ? 3 : 1);
 }
 
-// RanMars parity noise: both O-steps' normals of MD step h->step, from the
-// streams' current positions (the previous step's stay in the other half).
-static void draw_noise(pimdb_handle* h) {
+// RanMars parity noise: both O-steps' normals of MD step `step`, from the
+// streams' current positions (the step before's stay in the other half).
+static void draw_noise(pimdb_handle* h, long long step) {
     if (!h->d_noise) return;
     launch(h, PIMDB_K_CART_UPDATE, [&] {
-        launch_ranmars_draw(h->s, h->D, h->d_rng, h->d_noise, step_ref(h, h->step), h->stream);
+        launch_ranmars_draw(h->s, h->D, h->d_rng, h->d_noise, step_ref(h, step), h->stream);
     });
 }
 
@@ -863,17 +860,30 @@ static void enqueue_steps(pimdb_handle* h, int nsteps) {
     const pimdb_config& c = h->cfg;
     const bool nm = c.propagator == PIMDB_PROP_NORMAL_MODES;
     const bool cart_langevin = c.thermostat == PIMDB_THERMO_LANGEVIN && !c.nmthermostat;
+    // The last momentum update of a step with the Cartesian Langevin
+    // thermostat: B, O and, when another step follows, that step's first O in
+    // the same pass (COM O2, COM O1 = COM after both: the removal is a linear
+    // projection and O is affine).
+    auto kick_langevin = [&](bool more, int kick_nm) {
+        if (more) draw_noise(h, h->step + 1);
+        cart(h, SF_KICK | SF_LANGEVIN | (more ? SF_LANGEVIN_NEXT : 0) | (c.fixcom ? SF_COM_PARTIAL : 0), 1, kick_nm);
+    };
+    bool head_done = false;  // this step's first O was part of the previous step's last pass
     for (int it = 0; it < nsteps; ++it) {
-        draw_noise(h);
+        const bool more = it + 1 < nsteps;
         // O, [COM] (inside the fused normal-mode kernel when that is used)
-        if (!(nm && h->fused_nm)) thermostat_step(h, 0);
+        if (!head_done) {
+            draw_noise(h, h->step);
+            if (!(nm && h->fused_nm)) thermostat_step(h, 0);
+        }
         if (!nm) {
             // [COM], B, A (velocity_verlet.cpp:9-12)
             cart(h, SF_COM_APPLY | SF_KICK | SF_DRIFT, 0, 0);
             enqueue_forces(h);
             // B, then O (+ partials) when the thermostat is Cartesian Langevin
             if (cart_langevin) {
-                cart(h, SF_KICK | SF_LANGEVIN | (c.fixcom ? SF_COM_PARTIAL : 0), 1, 0);
+                kick_langevin(more, 0);
+                head_done = more;
             } else {
                 cart(h, SF_KICK, 1, 0);
                 thermostat_step(h, 1);
@@ -902,12 +912,13 @@ static void enqueue_steps(pimdb_handle* h, int nsteps) {
             const int apply = h->com_pending ? 1 : 0;
             launch(h, PIMDB_K_NM_PROPAGATE, [&] {
                 launch_nm_propagate(h->s, h->D, h->d_C, h->d_T, h->d_rot, apply, h->d_red[rin], h->nred_last,
-                                    h->opt_fft ? (const double2*)h->d_tw : nullptr, h->d_cm, h->stream);
-            }, apply ? 2 : 1);
+                                    h->opt_fft ? (const double2*)h->d_tw : nullptr, h->stream);
+            });
             h->com_pending = false;
             enqueue_forces(h);
             if (cart_langevin) {
-                cart(h, SF_KICK | SF_LANGEVIN | (c.fixcom ? SF_COM_PARTIAL : 0), 1, 1);
+                kick_langevin(more, 1);
+                head_done = more;
             } else {
                 cart(h, SF_KICK, 1, 1);
                 thermostat_step(h, 1);
@@ -1598,7 +1609,7 @@ extern "C" int pimdb_thermostat_step(pimdb_handle* h, int substep) {
     if (!h || substep < 0 || substep > 1) return PIMDB_ERR_ARG;
     const pimdb_config& c = h->cfg;
     complete_pending(h);  // finish the previous step's deferred work first
-    if (substep == 0) draw_noise(h);  // the step's normals, as the reference draws them
+    if (substep == 0) draw_noise(h, h->step);  // the step's normals, as the reference draws them
     if (c.thermostat >= PIMDB_THERMO_NOSE_HOOVER) nose_hoover(h);
     else if (c.thermostat == PIMDB_THERMO_LANGEVIN && c.nmthermostat) nm_thermo(h, 0, substep);
     else if (c.thermostat == PIMDB_THERMO_LANGEVIN) cart(h, SF_LANGEVIN, substep, 0);
@@ -1623,7 +1634,7 @@ extern "C" int pimdb_propagate(pimdb_handle* h) {
         h->modes_valid = false;
         launch(h, PIMDB_K_NM_PROPAGATE, [&] {
             launch_nm_propagate(h->s, h->D, h->d_C, h->d_T, h->d_rot, 0, h->d_red[0], 0,
-                                h->opt_fft ? (const double2*)h->d_tw : nullptr, h->d_cm, h->stream);
+                                h->opt_fft ? (const double2*)h->d_tw : nullptr, h->stream);
         });
         enqueue_forces(h);
         cart(h, SF_KICK, 0, 1);

@@ -9,8 +9,8 @@
 //
 // The centre-of-mass correction needs a sum over every bead and particle.
 // The kernel that last changed the momenta writes per-block partial sums
-// (`red_out`); the next kernel reduces them in a fixed order at start-up
-// (`red_in`), so the result is deterministic.
+// (`red_out`), which its last block or the next kernel (`red_in`) adds up in a
+// fixed order, so the result is deterministic.
 #include <algorithm>
 
 #include "common.cuh"
@@ -84,25 +84,85 @@ __global__ void k_state_out(Sys s, double* __restrict__ ox, double* __restrict__
     }
 }
 
+// The centre-of-mass sums of one launch: `part` (this thread's sums per axis)
+// to per-block slots red_out[3 blk + a].  Up to kComDirect blocks the next
+// kernel's blocks add the slots up themselves (com_mean).  With more, that sum
+// was most of k_cart_update (3072 slots at N = 4096, P = 128: 88 us a launch,
+// 14-51 us without), so the block that finishes last adds them, in order, and
+// leaves the mean momentum in red_out[3 nblk + a] (no waiting; the counter
+// behind it, red_out[3 nblk + 3], is back at 0 for the next launch).  At small
+// sizes its fence, atomic and second pass would cost more than they save.
+// A warp whose pairs all lie on one axis adds up that axis alone.
+constexpr int kComDirect = 512;
 template <int D>
-__device__ __forceinline__ void com_from_partials(const Sys& s, const double* red_in, int nred, double* cm,
-                                                  double* shred) {
-    double acc[3] = {0.0, 0.0, 0.0};
-    for (int k = threadIdx.x; k < nred; k += blockDim.x) {
-#pragma unroll
-        for (int a = 0; a < D; ++a) acc[a] += red_in[3 * k + a];
-    }
-    const double inv = 1.0 / ((double)s.N * (double)s.P);
-#pragma unroll
-    for (int a = 0; a < D; ++a) cm[a] = block_sum(acc[a], shred) * inv;
-}
-
-template <int D>
-__device__ __forceinline__ void com_write_partials(double* part, double* red_out, double* shred) {
+__device__ __forceinline__ void com_write(const Sys& s, const double* part, double* red_out, int blk, int nblk) {
+    __shared__ double sh[3][32];
+    __shared__ int is_last;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
     for (int a = 0; a < D; ++a) {
-        const double t = block_sum(part[a], shred);
-        if (threadIdx.x == 0) red_out[3 * blockIdx.x + a] = t;
+        const bool any = __any_sync(0xffffffffu, part[a] != 0.0);
+        const double t = any ? warp_sum(part[a]) : 0.0;
+        if (lane == 0) sh[a][w] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < D) {
+        double t = 0.0;
+        for (int k = 0; k < nw; ++k) t += sh[threadIdx.x][k];
+        red_out[3 * blk + threadIdx.x] = t;
+    }
+    if (nblk <= kComDirect) return;
+    __threadfence();
+    __syncthreads();
+    unsigned* ctr = reinterpret_cast<unsigned*>(red_out + 3 * (size_t)nblk + 3);
+    if (threadIdx.x == 0) is_last = atomicAdd(ctr, 1u) == (unsigned)(nblk - 1);
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    double acc[D];
+#pragma unroll
+    for (int a = 0; a < D; ++a) acc[a] = 0.0;
+    for (int k = threadIdx.x; k < nblk; k += blockDim.x)
+#pragma unroll
+        for (int a = 0; a < D; ++a) acc[a] += ((volatile const double*)red_out)[3 * k + a];
+    const double inv = 1.0 / ((double)s.N * (double)s.P);
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+        const double t = block_sum(acc[a], sh[0]) * inv;
+        if (threadIdx.x == 0) red_out[3 * (size_t)nblk + a] = t;
+    }
+    if (threadIdx.x == 0) *ctr = 0u;
+}
+// The mean momentum from the sums of the launch before, for the whole block.
+template <int D>
+__device__ __forceinline__ void com_mean(const Sys& s, const double* red_in, int nred, double* cm) {
+    if (nred > kComDirect) {
+#pragma unroll
+        for (int a = 0; a < D; ++a) cm[a] = red_in[3 * (size_t)nred + a];
+        return;
+    }
+    __shared__ double sh[3][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    double acc[D];
+#pragma unroll
+    for (int a = 0; a < D; ++a) acc[a] = 0.0;
+    for (int k = threadIdx.x; k < nred; k += blockDim.x)
+#pragma unroll
+        for (int a = 0; a < D; ++a) acc[a] += red_in[3 * k + a];
+    const int used = min(nw, (nred + 31) >> 5);  // the warps that hold slots
+    if (w < used)
+#pragma unroll
+        for (int a = 0; a < D; ++a) {
+            const double t = warp_sum(acc[a]);
+            if (lane == 0) sh[a][w] = t;
+        }
+    __syncthreads();
+    const double inv = 1.0 / ((double)s.N * (double)s.P);
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+        double t = 0.0;
+        for (int k = 0; k < used; ++k) t += sh[a][k];
+        cm[a] = t * inv;
     }
 }
 
@@ -121,44 +181,81 @@ __device__ __forceinline__ double nm_kick_force(const Sys& s, int b, int a, int 
     return fk;
 }
 
-// One thread per (bead, axis, particle pair).
-template <int D>
-__global__ void k_cart_update(Sys s, int flags, const double* __restrict__ red_in, int nred_in,
-                              double* __restrict__ red_out, StepRef sref, int substep, int kick_nm) {
+// K (bead, axis, particle pair)s per thread, a block's K 256 in a row; the
+// pair (2 i2, 2 i2 + 1) is one aligned 16-byte word of each array (for odd N
+// the last pair's second element is padding, stored back unchanged).
+constexpr int kCartThreads = 256;
+template <int D, int K>
+__global__ void __launch_bounds__(kCartThreads) k_cart_update(Sys s, int flags, const double* __restrict__ red_in,
+                                                              int nred_in, double* __restrict__ red_out, StepRef sref,
+                                                              int substep, int kick_nm) {
     const long long step = sref.get();
-    __shared__ double shred[32];
     const int half = (s.N + 1) / 2;
-    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const size_t total = (size_t)s.P * D * half;
+    const size_t t0 = blockIdx.x * (size_t)(K * kCartThreads) + threadIdx.x;
     double cm[3] = {0.0, 0.0, 0.0};
-    if (flags & SF_COM_APPLY) com_from_partials<D>(s, red_in, nred_in, cm, shred);
-    double part[3] = {0.0, 0.0, 0.0};
-    if (t < total) {
-        const int i2 = (int)(t % half);
-        const int ba = (int)(t / half);
-        const int a = ba % D;
-        const int b = ba / D;
-        double2 z = make_double2(0.0, 0.0);
-        if (flags & SF_LANGEVIN)
-            z = langevin_pair<D>(s, 2ull * (unsigned long long)step + substep, b, a, i2, half);
+    if (flags & SF_COM_APPLY) com_mean<D>(s, red_in, nred_in, cm);
+    double part[D];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int i = 2 * i2 + h;
-            if (i >= s.N) break;
-            const size_t o = idx<D>(s, b, a, i);
-            double p = s.p[o];
-            if (flags & SF_COM_APPLY) p -= cm[a];
-            if (flags & SF_KICK) {
-                const double fk = kick_nm ? nm_kick_force<D>(s, b, a, i) : s.f[o];
-                p += 0.5 * s.dt * fk;
-            }
-            if (flags & SF_LANGEVIN) p = s.c1 * p + s.c2 * (h == 0 ? z.x : z.y);
-            if (flags & SF_DRIFT) s.x[o] = fma(p, s.dt_m, s.x[o]);
-            s.p[o] = p;
-            part[a] += p;
+    for (int a = 0; a < D; ++a) part[a] = 0.0;
+    const double hdt = 0.5 * s.dt;
+    double2 pv[K], fv[K], xv[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const size_t t = t0 + k * kCartThreads;
+        if (t >= total) break;
+        const int i2 = (int)(t % half), ba = (int)(t / half), a = ba % D, b = ba / D;
+        const size_t o = idx<D>(s, b, a, 2 * i2);
+        pv[k] = *reinterpret_cast<const double2*>(s.p + o);
+        if (flags & SF_KICK) {
+            if (kick_nm)
+                fv[k] = make_double2(nm_kick_force<D>(s, b, a, 2 * i2),
+                                     2 * i2 + 1 < s.N ? nm_kick_force<D>(s, b, a, 2 * i2 + 1) : 0.0);
+            else
+                fv[k] = *reinterpret_cast<const double2*>(s.f + o);
+        }
+        if (flags & SF_DRIFT) xv[k] = *reinterpret_cast<const double2*>(s.x + o);
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const size_t t = t0 + k * kCartThreads;
+        if (t >= total) break;
+        const int i2 = (int)(t % half), ba = (int)(t / half), a = ba % D, b = ba / D;
+        const size_t o = idx<D>(s, b, a, 2 * i2);
+        const bool two = 2 * i2 + 1 < s.N;
+        double p0 = pv[k].x, p1 = pv[k].y;
+        if (flags & SF_COM_APPLY) {
+            const double c = a == 0 ? cm[0] : (a == 1 ? cm[1] : cm[2]);
+            p0 -= c;
+            p1 -= c;
+        }
+        if (flags & SF_KICK) {
+            p0 += hdt * fv[k].x;
+            p1 += hdt * fv[k].y;
+        }
+        if (flags & SF_LANGEVIN) {
+            const double2 z = langevin_pair<D>(s, 2ull * (unsigned long long)step + substep, b, a, i2, half);
+            p0 = s.c1 * p0 + s.c2 * z.x;
+            p1 = s.c1 * p1 + s.c2 * z.y;
+        }
+        if (flags & SF_LANGEVIN_NEXT) {
+            const double2 z = langevin_pair<D>(s, 2ull * (unsigned long long)(step + 1), b, a, i2, half);
+            p0 = s.c1 * p0 + s.c2 * z.x;
+            p1 = s.c1 * p1 + s.c2 * z.y;
+        }
+        if (!two) p1 = pv[k].y;  // padding: unchanged
+        if (flags & SF_DRIFT)
+            *reinterpret_cast<double2*>(s.x + o) =
+                make_double2(fma(p0, s.dt_m, xv[k].x), two ? fma(p1, s.dt_m, xv[k].y) : xv[k].y);
+        *reinterpret_cast<double2*>(s.p + o) = make_double2(p0, p1);
+        if (flags & SF_COM_PARTIAL) {
+            const double v = two ? p0 + p1 : p0;
+#pragma unroll
+            for (int c = 0; c < D; ++c)
+                if (a == c) part[c] += v;
         }
     }
-    if (flags & SF_COM_PARTIAL) com_write_partials<D>(part, red_out, shred);
+    if (flags & SF_COM_PARTIAL) com_write<D>(s, part, red_out, blockIdx.x, gridDim.x);
 }
 
 constexpr int kNmTile = 4;                           // particles per block
@@ -180,18 +277,21 @@ __global__ void __launch_bounds__(kNmThreads) k_nm_thermo(Sys s, const double* _
                                                           int substep) {
     const long long step = sref.get();
     extern __shared__ double sm[];
-    __shared__ double shred[32];
     const int P = s.P;
     double* sp = sm;                 // [P][kNmTile]
     double* sq = sm + P * kNmTile;   // [P][kNmTile]
     const int a = blockIdx.y;
     const int i0 = blockIdx.x * kNmTile;
     const int pp = threadIdx.x % kNmPairs, g = threadIdx.x / kNmPairs;
-    double cm[3] = {0.0, 0.0, 0.0};
-    if (flags & SF_COM_APPLY) com_from_partials<D>(s, red_in, nred_in, cm, shred);
+    double cms[D];
+    if (flags & SF_COM_APPLY) com_mean<D>(s, red_in, nred_in, cms);
+    double cm = 0.0;
+#pragma unroll
+    for (int c = 0; c < D; ++c)
+        if ((flags & SF_COM_APPLY) && c == a) cm = cms[c];
     for (int e = threadIdx.x; e < P * kNmTile; e += blockDim.x) {
         const int b = e / kNmTile, il = e % kNmTile, i = i0 + il;
-        sp[e] = i < s.N ? s.p[idx<D>(s, b, a, i)] - cm[a] : 0.0;
+        sp[e] = i < s.N ? s.p[idx<D>(s, b, a, i)] - cm : 0.0;
     }
     __syncthreads();
     const int half = (s.N + 1) / 2;
@@ -230,12 +330,10 @@ __global__ void __launch_bounds__(kNmThreads) k_nm_thermo(Sys s, const double* _
         }
     }
     if (flags & SF_COM_PARTIAL) {
-        const int bid = blockIdx.y * gridDim.x + blockIdx.x;
-        const double tsum = block_sum(part, shred);
-        if (threadIdx.x == 0) {
+        double sum[D];
 #pragma unroll
-            for (int ax = 0; ax < D; ++ax) red_out[3 * bid + ax] = ax == a ? tsum : 0.0;
-        }
+        for (int c = 0; c < D; ++c) sum[c] = c == a ? part : 0.0;
+        com_write<D>(s, sum, red_out, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y);
     }
 }
 
@@ -250,7 +348,6 @@ __global__ void __launch_bounds__(kNmThreads) k_nm_propagate(Sys s, const double
                                                              const double* __restrict__ rot, int com_apply,
                                                              const double* __restrict__ red_in, int nred_in) {
     extern __shared__ double sm[];
-    __shared__ double shred[32];
     const int P = s.P;
     double* sx = sm;
     double* sp = sm + P * kNmTile;
@@ -259,15 +356,19 @@ __global__ void __launch_bounds__(kNmThreads) k_nm_propagate(Sys s, const double
     const int a = blockIdx.y;
     const int i0 = blockIdx.x * kNmTile;
     const int pp = threadIdx.x % kNmPairs, g = threadIdx.x / kNmPairs;
-    double cm[3] = {0.0, 0.0, 0.0};
-    if (com_apply) com_from_partials<D>(s, red_in, nred_in, cm, shred);
+    double cms[D];
+    if (com_apply) com_mean<D>(s, red_in, nred_in, cms);
+    double cm = 0.0;
+#pragma unroll
+    for (int c = 0; c < D; ++c)
+        if (com_apply && c == a) cm = cms[c];
     for (int e = threadIdx.x; e < P * kNmTile; e += blockDim.x) {
         const int b = e / kNmTile, il = e % kNmTile, i = i0 + il;
         double x = 0.0, p = 0.0;
         if (i < s.N) {
             const size_t o = idx<D>(s, b, a, i);
             x = s.x[o];
-            p = s.p[o] - cm[a];
+            p = s.p[o] - cm;
             p += 0.5 * s.dt * nm_kick_force<D>(s, b, a, i);
         }
         sx[e] = x;
@@ -1101,50 +1202,68 @@ static bool nm_warp3_fits(const Sys& s) {
 
 // The normal-mode propagator's step (normal_modes_propagator.cpp:19-71:
 // [COM], half-kick, free ring rotation) with the transforms in registers,
-// for P = 32, 64, 128: two warps per (particle pair, axis), warp 0 on p and
-// warp 1 on x; they swap modes in shared memory for the rotation.  No grid
-// barrier: the pending COM correction comes reduced (`cmv`, or null).
+// for P = 32, 64, 128: two warps per (particle pair, axis), one on p and one
+// on x; they swap modes in shared memory for the rotation.  No grid barrier:
+// the pending COM correction comes from the sums before (`red_in`, or null).
+// A block takes
+// kNmPropPairs neighbouring pairs of an axis: a lane (one bead) reads and
+// writes a pair as one 16-byte word, and the block's pairs share the words'
+// 32-byte sectors.  Bound: the FP64 pipe (392 us at N = 4096, P = 128, about
+// 390 FP64 instructions a warp; the same with one pair per block).
+constexpr int kNmPropPairs = 2;
 template <int D, int E>
-__global__ void __launch_bounds__(64) k_nm_prop_warp(Sys s, const double* __restrict__ rot,
-                                                     const double* __restrict__ cmv,
-                                                     const double2* __restrict__ tw_g) {
+__global__ void __launch_bounds__(64 * kNmPropPairs) k_nm_prop_warp(Sys s, const double* __restrict__ rot,
+                                                                    const double* __restrict__ red_in, int nred_in,
+                                                                    const double2* __restrict__ tw_g) {
     constexpr int P = 32 * E;
     __shared__ double2 tw[P / 2];
-    __shared__ double2 sm2[2][E][32];  // [0] p modes, [1] x modes
+    __shared__ double2 sm2[kNmPropPairs][2][E][32];  // [0] p modes, [1] x modes
     for (int t = threadIdx.x; t < P / 2; t += blockDim.x) tw[t] = tw_g[t];
     __syncthreads();
-    const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;  // 0: p, 1: x
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, role = w & 1, pr = w >> 1;  // role 0: p, 1: x
     const int half = (s.N + 1) / 2;
-    const int u = blockIdx.x;
-    const int a = u / half, i2 = u % half;
-    const int ia = 2 * i2, ib = 2 * i2 + 1;
-    const bool va = ia < s.N, vb = ib < s.N;
-    const double cm = cmv ? cmv[a] : 0.0, hdt = 0.5 * s.dt;
+    const int a = blockIdx.y, i2 = blockIdx.x * kNmPropPairs + pr;
+    const int ia = 2 * i2;
+    const bool va = i2 < half, vb = ia + 1 < s.N;
+    double cms[D];
+    if (red_in) com_mean<D>(s, red_in, nred_in, cms);
+    double cm = 0.0;
+#pragma unroll
+    for (int c = 0; c < D; ++c)
+        if (red_in && c == a) cm = cms[c];
+    const double hdt = 0.5 * s.dt;
+    const double* src = role == 0 ? s.p : s.x;
     double2 z[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-        const int b = 32 * e + lane;
         z[e] = make_double2(0.0, 0.0);
-        if (va) {
-            const size_t o = idx<D>(s, b, a, ia);
-            z[e].x = role == 0 ? (s.p[o] - cm) + hdt * nm_kick_force<D>(s, b, a, ia) : s.x[o];
+        if (va) z[e] = *reinterpret_cast<const double2*>(src + idx<D>(s, 32 * e + lane, a, ia));
+    }
+    double pad[E];  // the padding beside an odd N's last particle, stored back unchanged
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int b = 32 * e + lane;
+        pad[e] = z[e].y;
+        if (role == 0 && va) {
+            double2 fk = *reinterpret_cast<const double2*>(s.fphys + idx<D>(s, b, a, ia));
+            if (s.bosonic && (b == 0 || b == P - 1))
+                fk = make_double2(nm_kick_force<D>(s, b, a, ia), vb ? nm_kick_force<D>(s, b, a, ia + 1) : 0.0);
+            z[e].x = (z[e].x - cm) + hdt * fk.x;
+            z[e].y = (z[e].y - cm) + hdt * fk.y;
         }
-        if (vb) {
-            const size_t o = idx<D>(s, b, a, ib);
-            z[e].y = role == 0 ? (s.p[o] - cm) + hdt * nm_kick_force<D>(s, b, a, ib) : s.x[o];
-        }
+        if (!vb) z[e].y = 0.0;
     }
     warp_fft_fwd<E>(z, tw, P, lane);
     warp_to_modes<E>(z, P, lane);
 #pragma unroll
-    for (int k1 = 0; k1 < E; ++k1) sm2[role][k1][lane] = z[k1];
+    for (int k1 = 0; k1 < E; ++k1) sm2[pr][role][k1][lane] = z[k1];
     __syncthreads();
     const int k2 = (int)(__brev((unsigned)lane) >> 27);
 #pragma unroll
     for (int k1 = 0; k1 < E; ++k1) {
         const int k = k1 + E * k2;
         const double cs = rot[4 * k], sn = rot[4 * k + 1], mw = rot[4 * k + 2], snw = rot[4 * k + 3];
-        const double2 pm = sm2[0][k1][lane], q = sm2[1][k1][lane];
+        const double2 pm = sm2[pr][0][k1][lane], q = sm2[pr][1][k1][lane];
         auto turn = [&](double q0, double p0) -> double {
             if (mw == 0.0) return role == 0 ? p0 : q0 + s.dt_m * p0;
             return role == 0 ? -mw * sn * q0 + cs * p0 : cs * q0 + snw * p0;
@@ -1153,23 +1272,12 @@ __global__ void __launch_bounds__(64) k_nm_prop_warp(Sys s, const double* __rest
     }
     warp_from_modes<E>(z, P, lane);
     warp_fft_inv<E>(z, tw, P, lane);
+    if (!va) return;
     double* dst = role == 0 ? s.p : s.x;
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const int b = 32 * e + lane;
-        if (va) dst[idx<D>(s, b, a, ia)] = z[e].x;
-        if (vb) dst[idx<D>(s, b, a, ib)] = z[e].y;
-    }
-}
-
-// The pending COM correction reduced once: cm[a] from the partial sums.
-template <int D>
-__global__ void k_com_mean(Sys s, const double* __restrict__ red_in, int nred, double* __restrict__ cm) {
-    __shared__ double shred[32];
-    double c[3] = {0.0, 0.0, 0.0};
-    com_from_partials<D>(s, red_in, nred, c, shred);
-    if (threadIdx.x == 0)
-        for (int a = 0; a < D; ++a) cm[a] = c[a];
+    for (int e = 0; e < E; ++e)
+        *reinterpret_cast<double2*>(dst + idx<D>(s, 32 * e + lane, a, ia)) =
+            make_double2(z[e].x, vb ? z[e].y : pad[e]);
 }
 
 // Warps per block of the warp kernel: the fewest (spreading the pairs over
@@ -1473,19 +1581,33 @@ void launch_state_out(const Sys& s, int D, double* ox, double* op, double* of, c
     else k_state_out<3><<<g, 256, 0, st>>>(s, ox, op, of);
 }
 
-int cart_update_blocks(const Sys& s, int D) {
+// Pairs per thread: four (their loads in flight together, the COM reduction
+// spread over them) once that still leaves two blocks per SM, else one.
+static int cart_pairs(const Sys& s, int D) {
     const size_t total = (size_t)s.P * D * ((s.N + 1) / 2);
-    return (int)((total + 255) / 256);
+    return total >= (size_t)4 * kCartThreads * 304 ? 4 : 1;
+}
+int cart_update_blocks(const Sys& s, int D) {
+    const size_t total = (size_t)s.P * D * ((s.N + 1) / 2), per = (size_t)kCartThreads * cart_pairs(s, D);
+    return (int)((total + per - 1) / per);
 }
 
 int nm_blocks(const Sys& s, int D) { return ((s.N + kNmTile - 1) / kNmTile) * D; }
 
+template <int D>
+static void cart_launch(const Sys& s, int flags, const double* red_in, int nred_in, double* red_out, StepRef step,
+                        int substep, int kick_nm, cudaStream_t st) {
+    const int g = cart_update_blocks(s, D);
+    if (cart_pairs(s, D) == 4)
+        k_cart_update<D, 4><<<g, kCartThreads, 0, st>>>(s, flags, red_in, nred_in, red_out, step, substep, kick_nm);
+    else
+        k_cart_update<D, 1><<<g, kCartThreads, 0, st>>>(s, flags, red_in, nred_in, red_out, step, substep, kick_nm);
+}
 void launch_cart_update(const Sys& s, int D, int flags, const double* red_in, int nred_in, double* red_out,
                         StepRef step, int substep, int kick_nm, cudaStream_t st) {
-    const int g = cart_update_blocks(s, D);
-    if (D == 1) k_cart_update<1><<<g, 256, 0, st>>>(s, flags, red_in, nred_in, red_out, step, substep, kick_nm);
-    else if (D == 2) k_cart_update<2><<<g, 256, 0, st>>>(s, flags, red_in, nred_in, red_out, step, substep, kick_nm);
-    else k_cart_update<3><<<g, 256, 0, st>>>(s, flags, red_in, nred_in, red_out, step, substep, kick_nm);
+    if (D == 1) cart_launch<1>(s, flags, red_in, nred_in, red_out, step, substep, kick_nm, st);
+    else if (D == 2) cart_launch<2>(s, flags, red_in, nred_in, red_out, step, substep, kick_nm, st);
+    else cart_launch<3>(s, flags, red_in, nred_in, red_out, step, substep, kick_nm, st);
 }
 
 template <int D>
@@ -1514,36 +1636,34 @@ static void nm_prop_launch(const Sys& s, const double* C, const double* T, const
 }
 
 template <int D, int E>
-static void nm_prop_warp_t(const Sys& s, const double* rot, int com_apply, const double* red_in, int nred_in,
-                           const double2* tw, double* cm, cudaStream_t st) {
-    if (com_apply) k_com_mean<D><<<1, 256, 0, st>>>(s, red_in, nred_in, cm);
-    const unsigned units = (unsigned)(D * ((s.N + 1) / 2));
-    k_nm_prop_warp<D, E><<<units, 64, 0, st>>>(s, rot, com_apply ? cm : nullptr, tw);
+static void nm_prop_warp_t(const Sys& s, const double* rot, const double* red_in, int nred_in, const double2* tw,
+                           cudaStream_t st) {
+    const dim3 grid(((s.N + 1) / 2 + kNmPropPairs - 1) / kNmPropPairs, D);
+    k_nm_prop_warp<D, E><<<grid, 64 * kNmPropPairs, 0, st>>>(s, rot, red_in, nred_in, tw);
 }
 
 template <int D>
-static bool nm_prop_warp_d(const Sys& s, const double* rot, int com_apply, const double* red_in, int nred_in,
-                           const double2* tw, double* cm, cudaStream_t st) {
-    if (s.P == 32) nm_prop_warp_t<D, 1>(s, rot, com_apply, red_in, nred_in, tw, cm, st);
-    else if (s.P == 64) nm_prop_warp_t<D, 2>(s, rot, com_apply, red_in, nred_in, tw, cm, st);
-    else if (s.P == 128) nm_prop_warp_t<D, 4>(s, rot, com_apply, red_in, nred_in, tw, cm, st);
+static bool nm_prop_warp_d(const Sys& s, const double* rot, const double* red_in, int nred_in, const double2* tw,
+                           cudaStream_t st) {
+    if (s.P == 32) nm_prop_warp_t<D, 1>(s, rot, red_in, nred_in, tw, st);
+    else if (s.P == 64) nm_prop_warp_t<D, 2>(s, rot, red_in, nred_in, tw, st);
+    else if (s.P == 128) nm_prop_warp_t<D, 4>(s, rot, red_in, nred_in, tw, st);
     else return false;
     return true;
 }
 
-int launch_nm_propagate(const Sys& s, int D, const double* C, const double* T, const double* rot, int com_apply,
-                        const double* red_in, int nred_in, const double2* tw, double* cm, cudaStream_t st) {
-    if (tw && cm) {
-        bool done = false;
-        if (D == 1) done = nm_prop_warp_d<1>(s, rot, com_apply, red_in, nred_in, tw, cm, st);
-        else if (D == 2) done = nm_prop_warp_d<2>(s, rot, com_apply, red_in, nred_in, tw, cm, st);
-        else done = nm_prop_warp_d<3>(s, rot, com_apply, red_in, nred_in, tw, cm, st);
-        if (done) return com_apply ? 2 : 1;
+void launch_nm_propagate(const Sys& s, int D, const double* C, const double* T, const double* rot, int com_apply,
+                         const double* red_in, int nred_in, const double2* tw, cudaStream_t st) {
+    if (tw) {
+        const double* red = com_apply ? red_in : nullptr;
+        if (D == 1 ? nm_prop_warp_d<1>(s, rot, red, nred_in, tw, st)
+                   : (D == 2 ? nm_prop_warp_d<2>(s, rot, red, nred_in, tw, st)
+                             : nm_prop_warp_d<3>(s, rot, red, nred_in, tw, st)))
+            return;
     }
     if (D == 1) nm_prop_launch<1>(s, C, T, rot, com_apply, red_in, nred_in, st);
     else if (D == 2) nm_prop_launch<2>(s, C, T, rot, com_apply, red_in, nred_in, st);
     else nm_prop_launch<3>(s, C, T, rot, com_apply, red_in, nred_in, st);
-    return 1;
 }
 
 }  // namespace pimdb

@@ -18,13 +18,17 @@ void nm_tables(int P, double omega_p, double mass, double dt, std::vector<double
 
 // Flags of the momentum-update kernels.  Within one launch the operations
 // run in this order: COM correction from the pending partial sums, B
-// half-kick, Langevin O-step, A drift, partial sums for the next COM removal.
+// half-kick, Langevin O-step(s), A drift, sums for the next COM removal.  The
+// sums: `red` buffers of com_doubles(nblocks) doubles, zeroed once.
 enum StepFlags : int {
     SF_COM_APPLY = 1,
     SF_LANGEVIN = 2,
     SF_COM_PARTIAL = 4,
     SF_KICK = 8,
     SF_DRIFT = 16,
+    // a second O-step, the first of the next MD step, right after this one's
+    // (O and the COM removal commute into one removal after both)
+    SF_LANGEVIN_NEXT = 32,
 };
 
 // forces.cu: external + pair forces and distinguishable springs on every
@@ -186,14 +190,14 @@ void launch_state_in(const Sys& s, int D, const double* sx, const double* sp, cu
 void launch_state_out(const Sys& s, int D, double* ox, double* op, double* of, cudaStream_t st);
 int cart_update_blocks(const Sys& s, int D);
 int nm_blocks(const Sys& s, int D);
+inline size_t com_doubles(int nblocks) { return 3 * (size_t)nblocks + 4; }
 void launch_cart_update(const Sys& s, int D, int flags, const double* red_in, int nred_in, double* red_out,
                         StepRef step, int substep, int kick_nm, cudaStream_t st);
 void launch_nm_thermo(const Sys& s, int D, const double* C, const double* T, int flags, const double* red_in,
                       int nred_in, double* red_out, StepRef step, int substep, cudaStream_t st);
-// With `tw` (FFT twiddles) and `cm` (3 doubles of scratch), P = 32, 64, 128
-// run the register-transform kernel; returns the number of kernels launched.
-int launch_nm_propagate(const Sys& s, int D, const double* C, const double* T, const double* rot, int com_apply,
-                        const double* red_in, int nred_in, const double2* tw, double* cm, cudaStream_t st);
+// With `tw` (FFT twiddles), P = 32, 64, 128 run the register-transform kernel.
+void launch_nm_propagate(const Sys& s, int D, const double* C, const double* T, const double* rot, int com_apply,
+                         const double* red_in, int nred_in, const double2* tw, cudaStream_t st);
 
 // Fused normal-mode step (normal-mode propagator + normal-mode Langevin):
 // mode bit 0 = tail of step-1 (kick, O, COM), bit 1 = head of step (O, COM,
