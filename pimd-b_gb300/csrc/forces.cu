@@ -263,6 +263,234 @@ __global__ void __launch_bounds__(128) k_pair_tiles(Sys s, double* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------
+// FP64 dipole pairs without a cutoff: near pairs in FP64, far ones in
+// double-float.  The gradient falls as r^-4, so beyond kFarRatio times its
+// nearest neighbour's distance a pair's force is at most kFarRatio^-4 = 2^-10
+// of the nearest one's, and its double-float evaluation (2^-44 of itself) adds
+// less than 2^-54 of what the nearest pair's own FP64 rounding leaves: the sum
+// over all far pairs keeps the FP64 result's accuracy at a seventh of the cost
+// per pair (about 130 FP32 operations against 15 FP64 ones at 1/64 the rate).
+// N = 1024, P = 32, 2D: 690 us with every pair in FP64 (k_pair_tiles, bound by
+// the FP64 pipe), 157 us and 17 us for the near radii so.
+// A pair is far when it is so for both its particles and its distance lies
+// where double-floats have room for r^-5; anything else, NaN included, is near.
+constexpr float kFarRatio2 = 36.0f;
+constexpr float kFarMinR2 = 1e-8f, kFarMaxR2 = 1e8f;
+constexpr int kNearFarWarps = 4;
+constexpr int kNearCap = 256;  // near gradients held per warp; a tile with more is summed in chunks
+
+// nr[b ld + i] = kFarRatio^2 min_j r_ij^2, from positions relative to the
+// bead's particle 0.
+template <int D>
+__global__ void __launch_bounds__(kPairThreads) k_near_radius(Sys s, float* __restrict__ nr) {
+    __shared__ float xs[D][kPairThreads];
+    const int b = blockIdx.y, i = blockIdx.x * kPairThreads + threadIdx.x;
+    double ref[D];
+    float xi[D];
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+        ref[a] = s.x[idx<D>(s, b, a, 0)];
+        xi[a] = i < s.N ? (float)(s.x[idx<D>(s, b, a, i)] - ref[a]) : 0.0f;
+    }
+    float best = INFINITY;
+    for (int j0 = 0; j0 < s.N; j0 += kPairThreads) {
+        const int jl = j0 + threadIdx.x;
+        __syncthreads();
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+            xs[a][threadIdx.x] = jl < s.N ? (float)(s.x[idx<D>(s, b, a, jl)] - ref[a]) : 0.0f;
+        __syncthreads();
+        const int jn = min(kPairThreads, s.N - j0);
+#pragma unroll 8
+        for (int jj = 0; jj < jn; ++jj) {
+            float r2 = 0.0f;
+#pragma unroll
+            for (int a = 0; a < D; ++a) {
+                const float d = xi[a] - xs[a][jj];
+                r2 = fmaf(d, d, r2);
+            }
+            if (j0 + jj != i) best = fminf(best, r2);
+        }
+    }
+    if (i < s.N) nr[(size_t)b * s.ld + i] = kFarRatio2 * best;
+}
+
+// |r|^-5 from r2 = |r|^2: y0 = rsqrtf(r2) has 24 bits, so y0^2 is exact in
+// FP64, e = 1 - r2 y0^2 is below 2^-21, and r^-5 = y0^5 (1 - e)^(-5/2) =
+// y0^5 (1 + 5/2 e + 35/8 e^2), the next term below 2^-60.  7 FP64 operations.
+__device__ __forceinline__ double inv_r5(double r2) {
+    const int hi = __double2hiint(r2);
+    if ((unsigned)hi - ((1023u - 100u) << 20) >= (200u << 20)) {  // beyond a float's exponents
+        const double y = rsqrt(r2), y2 = y * y;
+        return y2 * y2 * y;
+    }
+    const unsigned lo = (unsigned)__double2loint(r2);
+    const float y0f = rsqrtf(__int_as_float(((hi - ((1023 - 127) << 20)) << 3) | (int)(lo >> 29)));
+    const int yb = __float_as_int(y0f);
+    const double y0 = __hiloint2double((yb >> 3) + ((1023 - 127) << 20), yb << 29);
+    const double y2 = y0 * y0, e = fma(-r2, y2, 1.0);
+    const double y5 = (y2 * y2) * y0;
+    return fma(y5, e * fma(e, 4.375, 2.5), y5);
+}
+// The same in double-float (about 2^-45).
+__device__ __forceinline__ dfl::df inv_r5_df(dfl::df r2) {
+    const float y0 = rsqrtf(r2.hi);
+    const dfl::df y2 = dfl::two_prod(y0, y0), q = dfl::mul(r2, y2);
+    const float e = __fsub_rn(__fsub_rn(1.0f, q.hi), q.lo);
+    const dfl::df y4 = dfl::sqr(y2);
+    const dfl::df y5 = dfl::mul_f(y4, y0);
+    const float c = __fmul_rn(y5.hi, __fmul_rn(e, __fmaf_rn(e, 4.375f, 2.5f)));
+    return dfl::fast_two_sum(y5.hi, __fadd_rn(y5.lo, c));
+}
+
+template <int D>
+struct NearFarSmem {
+    double xi[kTile][D], xj[kTile][D];
+    double g[kNearCap][D];
+    unsigned mask[kTile];
+    int off[kTile];
+    unsigned short fe[kTile * kTile];
+};
+
+// One warp per tile pair, as k_pair_tiles: far pairs on the rotation, near
+// ones listed i-major and evaluated with every lane busy (as compact_tile).
+template <int D>
+__global__ void __launch_bounds__(32 * kNearFarWarps) k_pair_tiles_near_far(Sys s, double* __restrict__ part, int T,
+                                                                           int npairs, const float* __restrict__ nr) {
+    using dfl::df;
+    extern __shared__ __align__(16) unsigned char nf_raw[];
+    const int lane = threadIdx.x & 31, b = blockIdx.y;
+    const int w = blockIdx.x * kNearFarWarps + (threadIdx.x >> 5);
+    if (w >= npairs) return;
+    NearFarSmem<D>& sm = reinterpret_cast<NearFarSmem<D>*>(nf_raw)[threadIdx.x >> 5];
+    int it = 0, rem = w;
+    while (rem >= T - it) {
+        rem -= T - it;
+        ++it;
+    }
+    const int jt = it + rem;
+    const bool diag = it == jt;
+    const int i = it * kTile + lane, j = jt * kTile + lane;
+    df pi[D], pj[D];
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+        const double ref = s.x[idx<D>(s, b, a, 0)];
+        const double xv = i < s.N ? s.x[idx<D>(s, b, a, i)] : ref, yv = j < s.N ? s.x[idx<D>(s, b, a, j)] : ref;
+        sm.xi[lane][a] = xv;
+        sm.xj[lane][a] = yv;
+        pi[a] = split_df(xv - ref);
+        pj[a] = split_df(yv - ref);
+    }
+    const float ni = i < s.N ? nr[(size_t)b * s.ld + i] : 0.0f, njl = j < s.N ? nr[(size_t)b * s.ld + j] : 0.0f;
+    const int nj = min(kTile, s.N - jt * kTile);
+    df ai[D], aj[D];
+#pragma unroll
+    for (int a = 0; a < D; ++a) ai[a] = aj[a] = df{0.0f, 0.0f};
+    unsigned mask = 0u;
+    const int first = diag ? 1 : 0, lastS = diag ? 16 : 31;
+    // aj belongs to particle (lane + st) & 31 of tile jt and moves with it
+    for (int st = 0; st < 32; ++st) {
+        const int jl = (lane + st) & 31;
+        if (st >= first && st <= lastS) {
+            df d[D], r2;
+#pragma unroll
+            for (int a = 0; a < D; ++a) {
+                const df q{__shfl_sync(0xffffffffu, pj[a].hi, jl), __shfl_sync(0xffffffffu, pj[a].lo, jl)};
+                d[a] = dfl::add_sloppy(pi[a], dfl::neg(q));
+                r2 = a == 0 ? dfl::sqr(d[a]) : dfl::add_sloppy(r2, dfl::sqr(d[a]));
+            }
+            const float lim = fmaxf(ni, __shfl_sync(0xffffffffu, njl, jl));
+            const bool valid = i < s.N && jl < nj && (!diag || st < 16 || lane < 16);
+            const bool far = r2.hi >= lim && r2.hi >= kFarMinR2 && r2.hi <= kFarMaxR2;
+            mask |= (unsigned)(valid && !far) << jl;
+            if (valid && far) {
+                const df sc = inv_r5_df(r2);
+#pragma unroll
+                for (int a = 0; a < D; ++a) {
+                    const df v = dfl::mul(sc, d[a]);
+                    ai[a] = dfl::add_sloppy(ai[a], v);
+                    aj[a] = dfl::add_sloppy(aj[a], dfl::neg(v));
+                }
+            }
+        }
+        const int src = (lane + 1) & 31;
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+            aj[a] = df{__shfl_sync(0xffffffffu, aj[a].hi, src), __shfl_sync(0xffffffffu, aj[a].lo, src)};
+    }
+    // the near entries, i-major
+    const int icnt = __popc(mask);
+    int off = icnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, off, o);
+        if (lane >= o) off += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, off, 31);
+    off -= icnt;
+    sm.mask[lane] = mask;
+    sm.off[lane] = off;
+    {
+        unsigned mm = mask;
+        for (int f = off; mm; ++f) {
+            const int jj = __ffs(mm) - 1;
+            mm &= mm - 1u;
+            sm.fe[f] = (unsigned short)((lane << 5) | jj);
+        }
+    }
+    unsigned col = 0u;  // the i's whose masks hold bit `lane`
+#pragma unroll
+    for (int t = 0; t < 32; ++t) {
+        const unsigned bt = __ballot_sync(0xffffffffu, (mask >> t) & 1u);
+        if (lane == t) col = bt;
+    }
+    __syncwarp();
+    double fi[D], fj[D];
+#pragma unroll
+    for (int a = 0; a < D; ++a) fi[a] = fj[a] = 0.0;
+    const unsigned lt = (1u << lane) - 1u;
+    for (int c0 = 0; c0 < total; c0 += kNearCap) {
+        const int cend = min(total, c0 + kNearCap);
+        for (int f = c0 + lane; f < cend; f += 32) {
+            const int e = sm.fe[f], il = e >> 5, jl = e & 31;
+            double r[D], r2 = 0.0;
+#pragma unroll
+            for (int a = 0; a < D; ++a) {
+                r[a] = sm.xi[il][a] - sm.xj[jl][a];
+                r2 = a == 0 ? r[a] * r[a] : fma(r[a], r[a], r2);
+            }
+            const double sc = inv_r5(r2);
+#pragma unroll
+            for (int a = 0; a < D; ++a) sm.g[f - c0][a] = sc * r[a];
+        }
+        __syncwarp();
+        for (int k = max(off, c0); k < min(off + icnt, cend); ++k)
+#pragma unroll
+            for (int a = 0; a < D; ++a) fi[a] += sm.g[k - c0][a];
+        for (unsigned cm = col; cm; cm &= cm - 1u) {
+            const int ii = __ffs(cm) - 1, f = sm.off[ii] + __popc(sm.mask[ii] & lt);
+            if (f >= c0 && f < cend)
+#pragma unroll
+                for (int a = 0; a < D; ++a) fj[a] -= sm.g[f - c0][a];
+        }
+        __syncwarp();
+    }
+    // the force is 3 D_dip sum r^-5 r
+    const double k3 = 3.0 * s.int_a;
+    const size_t base_b = (size_t)b * T;
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+        const double vi = k3 * (fi[a] + df_to_f64(ai[a])), vj = k3 * (fj[a] + df_to_f64(aj[a]));
+        if (diag) {
+            if (i < s.N) part[((base_b + it) * D + a) * s.ld + i] = vi + vj;
+        } else {
+            if (i < s.N) part[((base_b + jt) * D + a) * s.ld + i] = vi;
+            if (j < s.N) part[((base_b + it) * D + a) * s.ld + j] = vj;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // FP64 pair tiles with lane compaction (plain path with a finite cutoff).
 // A warp-instruction on the FP64 pipe costs the same whether or not its lanes
 // are active, so evaluating the Aziz gradient only in the lanes whose pair is
@@ -1323,18 +1551,23 @@ void launch_pair_cells_and_finish(const Sys& s, int D, int nc, int mixed, int wr
     else cells_launch<3>(s, nc, mixed, write_phys, b, before_finish, add_fx, st);
 }
 
-// The partial sums plus one trailing double that holds the compact kernel's
-// two task counters (zero between launches).
-size_t pair_partial_doubles(const Sys& s, int D) {
-    const int T = (s.N + kTile - 1) / kTile;
-    return (size_t)s.P * T * D * s.ld + 1;
+// The partial sums, the near radii of the dipole tiles (floats) and one
+// trailing double that holds the compact kernel's two task counters (zero
+// between launches).
+static size_t pair_slot_doubles(const Sys& s, int D) {
+    return (size_t)s.P * ((s.N + kTile - 1) / kTile) * D * s.ld;
 }
+size_t pair_partial_doubles(const Sys& s, int D) { return pair_slot_doubles(s, D) + (size_t)s.P * s.ld / 2 + 1; }
 
 // Kernels of launch_pair_tiles_and_finish: without pairs, or with the
 // harmonic interaction of every pair in FP64 (O(N), in the finishing kernel;
 // mixed precision keeps its FP32 pair arithmetic), only the finishing one.
+static bool near_far_tiles(const Sys& s, int mixed) {
+    return !mixed && s.int_kind == POT_DIPOLE && s.cutoff < 0.0 && !s.pbc;
+}
 int pair_tile_kernels(const Sys& s, int mixed) {
     if (s.int_kind == POT_FREE || s.cutoff == 0.0) return 1;
+    if (near_far_tiles(s, mixed)) return 3;
     return !mixed && s.int_kind == POT_HARMONIC && s.cutoff < 0.0 && !s.pbc ? 1 : 2;
 }
 
@@ -1398,6 +1631,14 @@ static void tiles_launch(const Sys& s, int mixed, int write_phys, double* part, 
         const int np = T * (T + 1) / 2;
         if (s.cutoff > 0.0) {
             compact_launch<D>(s, mixed, part, T, nullptr, st);
+        } else if (near_far_tiles(s, mixed)) {
+            float* nr = reinterpret_cast<float*>(part + pair_slot_doubles(s, D));
+            const size_t smem = kNearFarWarps * sizeof(NearFarSmem<D>);
+            if (smem > 40 * 1024)
+                cudaFuncSetAttribute(k_pair_tiles_near_far<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            k_near_radius<D><<<dim3((s.N + kPairThreads - 1) / kPairThreads, s.P), kPairThreads, 0, st>>>(s, nr);
+            k_pair_tiles_near_far<D><<<dim3((np + kNearFarWarps - 1) / kNearFarWarps, s.P), 32 * kNearFarWarps, smem,
+                                      st>>>(s, part, T, np, nr);
         } else {
             dim3 grid((np + 3) / 4, s.P);
             if (mixed) k_pair_tiles<D, float><<<grid, 128, 0, st>>>(s, part, T, np);
