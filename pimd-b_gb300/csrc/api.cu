@@ -702,7 +702,7 @@ static void exchange_front(pimdb_handle* h, cudaStream_t st) {
     if (h->factorial) return;
     int est = 0;
     launch(h, PIMDB_K_EXCH_ENERGIES, [&] { est = launch_exchange_energies(s, h->D, st, h->d_ework); },
-           h->d_ework ? 2 : 1);
+           h->d_ework && s.eflat ? 3 : 1);
     const int ex = h->opt_exact_exchange;
     int nk = 0;
     launch(h, PIMDB_K_EXCH_RECURSIONS,

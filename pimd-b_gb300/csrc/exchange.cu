@@ -191,8 +191,10 @@ static bool energies_by_rows(const Sys& s, const double* work) {
 // sums L[w] = sum_{t<w} |x1_{t+1} - xP_t|^2 of the interior links, so every
 // entry is independent.  L is kept in double-double (hi, lo): the difference
 // of two long prefix sums then keeps the accuracy of the direct sum.
-// k_link_prefix (one block) builds L and the beads' positions wrapped into
-// the box; k_exch_energies_flat (one block per row) writes E and Et.
+// k_link_prefix (one link per thread) scans blocks of kLinkBlock links and
+// wraps the beads' positions into the box, k_link_carry adds the blocks before
+// to each block's sums (on one block the whole scan was one SM's FP64 pipe:
+// 104 us at N = 4096, 9 + 6 us so), and k_exch_energies_flat writes E and Et.
 __device__ __forceinline__ void dd_add(double ah, double al, double bh, double bl, double& h, double& l) {
     const double s = ah + bh;
     const double bb = s - ah;
@@ -202,35 +204,31 @@ __device__ __forceinline__ void dd_add(double ah, double al, double bh, double b
     l = e - (h - s);
 }
 
+constexpr int kLinkBlock = 128;
+static int link_blocks(int N) { return (N + kLinkBlock - 1) / kLinkBlock; }
+
+// Lh, Ll: exclusive prefix of the link within its block; tot: the blocks' sums.
 template <int D>
-__global__ void __launch_bounds__(1024) k_link_prefix(Sys s, double* __restrict__ Lh, double* __restrict__ Ll,
-                                                       double* __restrict__ wrap) {
-    __shared__ double sh[32], sl[32];
-    const int N = s.N, tid = threadIdx.x, nt = blockDim.x;
+__global__ void __launch_bounds__(kLinkBlock) k_link_prefix(Sys s, double* __restrict__ Lh, double* __restrict__ Ll,
+                                                            double* __restrict__ wrap, double* __restrict__ tot) {
+    __shared__ double sh[kLinkBlock / 32], sl[kLinkBlock / 32];
+    const int N = s.N, tid = threadIdx.x, w = blockIdx.x * kLinkBlock + tid;
     const int first = 0, last = s.P - 1;
     // positions of beads 1 and P wrapped into [-L/2, L/2): wrap[side][a][N]
-    for (int i = tid; i < N; i += nt)
+    if (w < N)
 #pragma unroll
         for (int a = 0; a < D; ++a) {
-            double x1 = s.x[idx<D>(s, first, a, i)], xP = s.x[idx<D>(s, last, a, i)];
+            double x1 = s.x[idx<D>(s, first, a, w)], xP = s.x[idx<D>(s, last, a, w)];
             if (s.pbc) {
                 x1 -= s.L * rint(x1 * s.invL);
                 xP -= s.L * rint(xP * s.invL);
             }
-            wrap[(size_t)a * N + i] = x1;
-            wrap[(size_t)(D + a) * N + i] = xP;
+            wrap[(size_t)a * N + w] = x1;
+            wrap[(size_t)(D + a) * N + w] = xP;
         }
-    // contiguous chunk per thread, double-double sums, then a scan of the chunks
-    const int chunk = (N + nt - 1) / nt;
-    const int w0 = tid * chunk, w1 = min(N, w0 + chunk);
-    double th = 0.0, tl = 0.0;
-    for (int w = w0; w < w1 && w + 1 <= N - 1; ++w) {
-        double d2 = sepsq<D>(s, last, w, first, w + 1);
-        dd_add(th, tl, d2, 0.0, th, tl);
-    }
-    // inclusive warp scan, then across warps
+    // inclusive scan of the block's links in double-double: warps, then across
+    double ih = w + 1 <= N - 1 ? sepsq<D>(s, last, w, first, w + 1) : 0.0, il = 0.0;
     const int lane = tid & 31, warp = tid >> 5;
-    double ih = th, il = tl;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const double yh = __shfl_up_sync(0xffffffffu, ih, o), yl = __shfl_up_sync(0xffffffffu, il, o);
@@ -241,63 +239,134 @@ __global__ void __launch_bounds__(1024) k_link_prefix(Sys s, double* __restrict_
         sl[warp] = il;
     }
     __syncthreads();
-    if (warp == 0) {
-        double wh = lane < nt / 32 ? sh[lane] : 0.0, wl = lane < nt / 32 ? sl[lane] : 0.0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double yh = __shfl_up_sync(0xffffffffu, wh, o), yl = __shfl_up_sync(0xffffffffu, wl, o);
-            if (lane >= o) dd_add(yh, yl, wh, wl, wh, wl);
-        }
-        sh[lane] = wh;
-        sl[lane] = wl;
-    }
-    __syncthreads();
-    // exclusive prefix of this thread's chunk
     double ph = 0.0, pl = 0.0;
-    if (warp > 0) {
-        ph = sh[warp - 1];
-        pl = sl[warp - 1];
-    }
+    for (int k = 0; k < warp; ++k) dd_add(ph, pl, sh[k], sl[k], ph, pl);
+    if (tid == kLinkBlock - 1) dd_add(ph, pl, ih, il, tot[2 * blockIdx.x], tot[2 * blockIdx.x + 1]);
     const double xh = __shfl_up_sync(0xffffffffu, ih, 1), xl = __shfl_up_sync(0xffffffffu, il, 1);
     if (lane > 0) dd_add(ph, pl, xh, xl, ph, pl);
-    for (int w = w0; w < w1; ++w) {
+    if (w < N) {
         Lh[w] = ph;
         Ll[w] = pl;
-        if (w + 1 <= N - 1) {
-            const double d2 = sepsq<D>(s, last, w, first, w + 1);
-            dd_add(ph, pl, d2, 0.0, ph, pl);
-        }
+    }
+}
+__global__ void __launch_bounds__(kLinkBlock) k_link_carry(int N, double* __restrict__ Lh, double* __restrict__ Ll,
+                                                           const double* __restrict__ tot) {
+    const int w = blockIdx.x * kLinkBlock + threadIdx.x, lane = threadIdx.x & 31;
+    // the sum of the blocks before, by every warp alike
+    double ch = 0.0, cl = 0.0;
+    for (int k = lane; k < (int)blockIdx.x; k += 32) dd_add(ch, cl, tot[2 * k], tot[2 * k + 1], ch, cl);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double yh = __shfl_xor_sync(0xffffffffu, ch, o), yl = __shfl_xor_sync(0xffffffffu, cl, o);
+        dd_add(ch, cl, yh, yl, ch, cl);
+    }
+    if (w < N) dd_add(ch, cl, Lh[w], Ll[w], Lh[w], Ll[w]);
+}
+
+// The lower triangle in tiles of 16 rows and 32 columns (row tiles 2k and
+// 2k + 1 have k + 1 column tiles each), row-major: those of the flat energies
+// and of the weights, whose second copies (Et, Wb) are packed by column.  A
+// tile's transposed entries go through shared memory, so that the second copy
+// is written in runs of 16 entries (from the rows directly every entry was a
+// 32-byte sector of its own).
+constexpr int kTileRows = 16, kTileCols = 32, kTileThreads = 128;
+constexpr int kTileWarps = kTileThreads / 32, kTilePer = kTileRows / kTileWarps;  // rows per warp
+__device__ __forceinline__ void tile_of(int t, int& v0, int& u0) {
+    int k = (int)((sqrtf(4.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while ((k + 1) * (k + 2) <= t) ++k;
+    while (k * (k + 1) > t) --k;
+    const int r = t - k * (k + 1), odd = r > k;
+    v0 = kTileRows * (2 * k + odd);
+    u0 = kTileCols * (r - odd * (k + 1));
+}
+static int tile_count(int N) {
+    const int M = (N + kTileRows - 1) / kTileRows, k = M / 2;
+    return k * (k + 1) + (M & 1) * (k + 1);
+}
+// One tile's second copy: entry (v, u), u >= 1, to out[tri(N - u - 1) + N - 1 - v].
+__device__ __forceinline__ void tile_transposed(const double (*tile)[kTileCols + 1], int v0, int u0, int N,
+                                                double* __restrict__ out) {
+    const int row = threadIdx.x & (kTileRows - 1), c0 = threadIdx.x / kTileRows;
+#pragma unroll
+    for (int k = 0; k < kTileCols * kTileRows / kTileThreads; ++k) {
+        const int c = c0 + k * (kTileThreads / kTileRows), u = u0 + c, v = v0 + row;
+        if (u >= 1 && u <= v && v < N) out[tri(N - u - 1) + (N - 1 - v)] = tile[row][c];
     }
 }
 
+// E and Et from the prefix sums.  Under PBC the image of x1_u nearest to xP_v
+// is chosen on FP32 differences: xP_v minus x1_u + L, x1_u or x1_u - L, each
+// rounded once per tile; within 1e-6 L of the half-box edge, where FP32 might
+// choose the other image, by the FP64 difference.  Bound: the FP64 pipe, 11
+// operations an entry (3D): 302 -> 253 us at N = 4096, 19 -> 13 us at N = 777
+// against one block per row with the image taken from the FP64 difference.
 template <int D>
-__global__ void __launch_bounds__(256) k_exch_energies_flat(Sys s, const double* __restrict__ Lh,
-                                                            const double* __restrict__ Ll,
-                                                            const double* __restrict__ wrap) {
-    const int N = s.N, v = blockIdx.x;
+__global__ void __launch_bounds__(kTileThreads) k_exch_energies_flat(Sys s, const double* __restrict__ Lh,
+                                                                     const double* __restrict__ Ll,
+                                                                     const double* __restrict__ wrap) {
+    __shared__ double tile[kTileRows][kTileCols + 1];
+    const int N = s.N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int v0, u0;
+    tile_of(blockIdx.x, v0, u0);
+    const int u = u0 + lane;
     const double hk = 0.5 * s.kappa;
-    const long long half_bits = __double_as_longlong(0.5 * s.L);
-    double xv[D];
+    const float Lf = round_f32(s.L), halfLf = 0.5f * Lf, amb = 1e-6f * Lf;
+    double xu[D], xup[D], xum[D];
+    float xuf[D];
+    double luh = 0.0, lul = 0.0;
 #pragma unroll
-    for (int a = 0; a < D; ++a) xv[a] = wrap[(size_t)(D + a) * N + v];
-    const double lvh = Lh[v], lvl = Ll[v];
-    double* row = s.E + tri(v);
-    for (int u = threadIdx.x; u <= v; u += blockDim.x) {
+    for (int a = 0; a < D; ++a) {
+        xu[a] = u < N ? wrap[(size_t)a * N + u] : 0.0;
+        xuf[a] = round_f32(xu[a]);
+        xup[a] = xum[a] = xu[a];
+        if (s.pbc) {
+            xup[a] += s.L;
+            xum[a] -= s.L;
+        }
+    }
+    if (u < N) {
+        luh = Lh[u];
+        lul = Ll[u];
+    }
+    // the warp's rows, their values loaded together
+    double xv[kTilePer][D], lvh[kTilePer], lvl[kTilePer];
+#pragma unroll
+    for (int k = 0; k < kTilePer; ++k) {
+        const int v = min(v0 + warp + kTileWarps * k, N - 1);
+#pragma unroll
+        for (int a = 0; a < D; ++a) xv[k][a] = wrap[(size_t)(D + a) * N + v];
+        lvh[k] = Lh[v];
+        lvl[k] = Ll[v];
+    }
+#pragma unroll
+    for (int k = 0; k < kTilePer; ++k) {
+        const int r = warp + kTileWarps * k, v = v0 + r;
+        if (v >= N) break;  // rows ascend: uniform in the warp
         double c = 0.0;
 #pragma unroll
         for (int a = 0; a < D; ++a) {
-            double d = xv[a] - wrap[(size_t)a * N + u];
+            double d;
             if (s.pbc) {
-                const long long bits = __double_as_longlong(d);
-                if ((bits & 0x7fffffffffffffffLL) > half_bits) d -= copysign(s.L, d);
+                const float df = round_f32(xv[k][a]) - xuf[a];
+                const float over = fabsf(df) - halfLf;
+                const double im = over > 0.0f ? (df > 0.0f ? xup[a] : xum[a]) : xu[a];
+                d = xv[k][a] - im;
+                if (fabsf(over) <= amb) {
+                    d = xv[k][a] - xu[a];
+                    if (fabs(d) > 0.5 * s.L) d -= copysign(s.L, d);
+                }
+            } else {
+                d = xv[k][a] - xu[a];
             }
-            c = fma(d, d, c);
+            c = a == 0 ? d * d : fma(d, d, c);
         }
-        const double e = hk * (((lvh - Lh[u]) + (lvl - Ll[u])) + c);
-        row[u] = e;
-        // backward node r = N - u depends on node r' = N - 1 - v
-        if (u >= 1) s.Et[tri(N - u - 1) + (N - 1 - v)] = e;
+        const double e = hk * (((lvh[k] - luh) + (lvl[k] - lul)) + c);
+        if (u <= v) s.E[tri(v) + u] = e;
+        tile[r][lane] = e;
     }
+    __syncthreads();
+    // backward node r = N - u depends on node r' = N - 1 - v
+    tile_transposed(tile, v0, u0, N, s.Et);
 }
 
 // Pass 1: block 0 forward, block 1 backward.  Phase 0 skips (early exit)
@@ -432,23 +501,64 @@ __global__ void __launch_bounds__(kGridSolveThreads) k_exch_estimate_grid(Sys s,
     }
 }
 
-// Pass 2: every FP64 exponential at once, one thread per packed entry
-// (grid-stride over rows; phase 1 runs only on a retry).
-// Also records the band of the weights (kExchBand: the largest p + 1 - u of
-// a nonzero weight) for the banded solve; one atomic per warp.
-__global__ void k_exch_weights(Sys s, int phase) {
+// Pass 2: every FP64 exponential at once, by tiles (grid-stride; phase 1 runs
+// only on a retry).  Also records the band of the weights (kExchBand: the
+// largest p + 1 - u of a nonzero weight) for the banded solve; one atomic per
+// warp.  An entry whose FP32 argument, with the roundings of E and the two
+// potentials added, is below -701 is exactly zero (exp_tang's) without any
+// FP64 operation: nearly all of them in a large liquid (N = 4096: 245 -> 114 us
+// against one row per block without the test; where no entry is zero the FP64
+// pipe bounds either form, 23 -> 34 us at N = 777).
+__global__ void __launch_bounds__(kTileThreads) k_exch_weights(Sys s, int phase, int tiles) {
     if (phase == 1 && ((volatile int*)s.xflags)[6] == 0) return;
     __shared__ double tbl[32];
+    __shared__ double tile[kTileRows][kTileCols + 1];
     if (threadIdx.x < 32) tbl[threadIdx.x] = kExp2Table[threadIdx.x];
     __syncthreads();
+    const int N = s.N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double beta = s.beta_ex;
+    const float bf = round_f32(beta);
+    // whether w = exp(-beta (E + a - b)) / (p + 1) can be other than zero
+    auto live = [&](float E, float a, float b) {
+        return !(-(E + (a - b)) + 4e-7f * (fabsf(E) + fabsf(a) + fabsf(b)) < -701.0f);
+    };
     int band = 0;
-    for (int p = blockIdx.y; p < s.N; p += gridDim.y) {
-        const double inv = recip_row(p);
-        for (int u = blockIdx.x * blockDim.x + threadIdx.x; u <= p; u += gridDim.x * blockDim.x)
-            if (exch_weight(s, p, u, inv, tbl)) band = max(band, p + 1 - u);
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+        int p0, u0;
+        tile_of(t, p0, u0);
+        const int u = u0 + lane;
+        const double vu = u < N ? s.Vh[u] : 0.0, vbu = u < N ? s.Vbh[u] : 0.0;
+        double E[kTilePer];
+#pragma unroll
+        for (int k = 0; k < kTilePer; ++k) {
+            const int p = p0 + warp + kTileWarps * k;
+            E[k] = p < N && u <= p ? s.E[tri(p) + u] : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < kTilePer; ++k) {
+            const int r = warp + kTileWarps * k, p = p0 + r;
+            if (p >= N) break;
+            const double vp = s.Vh[p + 1], vbp = s.Vbh[p + 1];
+            const float ef = bf * round_f32(E[k]);
+            const bool lf = u <= p && live(ef, bf * round_f32(vu), bf * round_f32(vp));
+            // backward node r = N - u from node r' = N - 1 - p (u >= 1)
+            const bool lb = u <= p && u >= 1 && live(ef, bf * round_f32(vbp), bf * round_f32(vbu));
+            double wf = 0.0, wb = 0.0;
+            if (__any_sync(0xffffffffu, lf || lb)) {  // the warp's FP64 part, or none of it
+                const double inv = recip_row(p);
+                if (lf) wf = weight_exp(-beta * (E[k] + vu - vp), tbl) * inv;
+                if (lb) wb = weight_exp(-beta * (E[k] + vbp - vbu), tbl) * inv;
+                if (!f64_is_zero(wf) || !f64_is_zero(wb)) band = max(band, p + 1 - u);
+            }
+            if (u <= p) s.Wf[tri(p) + u] = wf;
+            tile[r][lane] = wb;
+        }
+        __syncthreads();
+        tile_transposed(tile, p0, u0, N, s.Wb);
+        __syncthreads();
     }
     band = __reduce_max_sync(0xffffffffu, band);
-    if ((threadIdx.x & 31) == 0 && band > 0) atomicMax(&s.xflags[kExchBand], band);
+    if (lane == 0 && band > 0) atomicMax(&s.xflags[kExchBand], band);
 }
 
 // Pass 3: block 0 forward, block 1 backward.  Phase 0 may not fall back to
@@ -894,7 +1004,7 @@ static void exchange_carveouts() {
     const void* k[] = {(const void*)k_exch_energies<1>, (const void*)k_exch_energies<2>,
                        (const void*)k_exch_energies<3>, (const void*)k_exch_energies_rows<1>,
                        (const void*)k_exch_energies_rows<2>, (const void*)k_exch_energies_rows<3>, (const void*)k_link_prefix<1>,
-                       (const void*)k_link_prefix<2>, (const void*)k_link_prefix<3>,
+                       (const void*)k_link_prefix<2>, (const void*)k_link_prefix<3>, (const void*)k_link_carry,
                        (const void*)k_exch_energies_flat<1>, (const void*)k_exch_energies_flat<2>,
                        (const void*)k_exch_energies_flat<3>, (const void*)k_exch_estimate, (const void*)k_exch_estimate_grid,
                        (const void*)k_exch_weights, (const void*)k_exch_solve, (const void*)k_exch_solve_grid,
@@ -916,25 +1026,28 @@ static void opt_in_smem(const void* k, size_t dyn) {
     if (dyn + kSmemOptInMargin > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
 }
 
-// The work array of the prefix-sum energies (any N: Sys::eflat chooses).
-size_t exchange_energy_doubles(const Sys& s, int D) { return (size_t)(2 + 2 * D) * s.N; }
+// The work array of the prefix-sum energies (any N: Sys::eflat chooses): the
+// prefix sums, the wrapped positions, the blocks' sums.
+size_t exchange_energy_doubles(const Sys& s, int D) { return (size_t)(2 + 2 * D) * s.N + 2 * (size_t)link_blocks(s.N); }
+
+template <int D>
+static void flat_launch(const Sys& s, double* work, cudaStream_t st) {
+    const int nb = link_blocks(s.N);
+    double* Lh = work;
+    double* Ll = work + s.N;
+    double* wrap = work + 2 * (size_t)s.N;
+    double* tot = wrap + (size_t)2 * D * s.N;
+    k_link_prefix<D><<<nb, kLinkBlock, 0, st>>>(s, Lh, Ll, wrap, tot);
+    if (nb > 1) k_link_carry<<<nb, kLinkBlock, 0, st>>>(s.N, Lh, Ll, tot);
+    k_exch_energies_flat<D><<<tile_count(s.N), kTileThreads, 0, st>>>(s, Lh, Ll, wrap);
+}
 
 int launch_exchange_energies(const Sys& s, int D, cudaStream_t st, double* work) {
     exchange_carveouts();
     if (work && s.eflat) {
-        double* Lh = work;
-        double* Ll = work + s.N;
-        double* wrap = work + 2 * (size_t)s.N;
-        if (D == 1) {
-            k_link_prefix<1><<<1, 1024, 0, st>>>(s, Lh, Ll, wrap);
-            k_exch_energies_flat<1><<<s.N, 256, 0, st>>>(s, Lh, Ll, wrap);
-        } else if (D == 2) {
-            k_link_prefix<2><<<1, 1024, 0, st>>>(s, Lh, Ll, wrap);
-            k_exch_energies_flat<2><<<s.N, 256, 0, st>>>(s, Lh, Ll, wrap);
-        } else {
-            k_link_prefix<3><<<1, 1024, 0, st>>>(s, Lh, Ll, wrap);
-            k_exch_energies_flat<3><<<s.N, 256, 0, st>>>(s, Lh, Ll, wrap);
-        }
+        if (D == 1) flat_launch<1>(s, work, st);
+        else if (D == 2) flat_launch<2>(s, work, st);
+        else flat_launch<3>(s, work, st);
         return 0;
     }
     // one block per row; scans [N] and two chunk arrays in shared memory
@@ -1025,8 +1138,7 @@ int launch_exchange_recursions(const Sys& s, int exact, cudaStream_t st, double*
         k_exch_solve<<<2, kWaveThreads, smem, st>>>(s, 1, 0, nullptr, 0);
         return 1;
     }
-    const dim3 wgrid((s.N + 255) / 256, s.N < 65535 ? s.N : 65535);
-    const dim3 rgrid(1, s.N < 256 ? s.N : 256);  // the retry's weights: a small grid-stride launch
+    const int tiles = tile_count(s.N);  // the retry's weights: a small grid-stride launch
     // below the multi-SM solve's size a failed solve is retried inside
     // k_exch_solve (phase 0 only)
     const int inline_retry = s.N < kGridSolveMinN;
@@ -1041,7 +1153,7 @@ int launch_exchange_recursions(const Sys& s, int exact, cudaStream_t st, double*
             ++n;
         }
         if (!(phase == 0 && estimate_done)) {  // else the energy kernel formed them
-            k_exch_weights<<<phase ? rgrid : wgrid, 256, 0, st>>>(s, phase);
+            k_exch_weights<<<phase ? std::min(tiles, 512) : tiles, kTileThreads, 0, st>>>(s, phase, tiles);
             ++n;
         }
         // the banded kernel (one CTA per direction): below the multi-SM
