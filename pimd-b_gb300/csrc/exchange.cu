@@ -770,23 +770,104 @@ __global__ void __launch_bounds__(kGridSolveThreads) k_exch_solve_grid(Sys s, in
 // (blocked_solve), a reused estimate that fails is redone from a fresh one
 // in the block (k_exch_solve's in-block retry), and the CTA that finishes
 // second runs solve_finish; no other solve kernel is launched.
+// solve_direction's post-processing of an inexact solve (y in shared memory),
+// with one pass over the nodes and one barrier: V or V_backwards, yf / yb and
+// the direction's flags.  Returns 1 (block-uniform, the flags untouched) where
+// the estimate proves unusable.  `word`: shared scratch.
+__device__ __forceinline__ int finish_direction(const Sys& s, int dir, const double* ys, const dfl::ExpTable& et,
+                                                int* word) {
+    const int N = s.N, tid = threadIdx.x, bd = blockDim.x;
+    if (tid == 0) *word = 0;
+    __syncthreads();
+    const double* Vh = dir == 0 ? s.Vh : s.Vbh;
+    double* V = dir == 0 ? s.V : s.Vb;
+    double* yo = dir == 0 ? s.yf : s.yb;
+    int flags = 0;  // 1 unusable, 2 thirty kT off, 4 not finite
+    for (int m = dir == 0 ? tid : tid + 1; m < N + (dir == 0); m += bd) {
+        const double y = ys[dir == 0 ? m : N - m];
+        const double ly = log_df(y, et);
+        const double v = Vh[m] - ly * s.inv_beta_ex;
+        if (!(y > 0.0) || !(fabs(ly) < kExactLogY)) flags |= 1;
+        if (!(fabs(ly) < kRefreshLogY)) flags |= 2;
+        if (!isfinite(v)) flags |= 4;
+        yo[m] = y;
+        V[m] = v;
+    }
+    if (dir == 1 && tid == 0) {
+        V[N] = 0.0;
+        yo[N] = 1.0;
+    }
+    if (flags) atomicOr(word, flags);
+    __syncthreads();
+    flags = *word;
+    __syncthreads();
+    if (flags & 1) return 1;
+    if (tid == 0) {
+        s.xflags[dir] = 0;
+        s.xflags[4 + dir] = flags >> 1;
+        if (flags & 4) atomicOr(s.err, ERRB_NONFINITE_VB);
+    }
+    return 0;
+}
+// solve_finish with every load issued at once: node m's row factors and next
+// estimate are one thread's.
+__device__ __forceinline__ void finish_both(const Sys& s, int extrapolate, const dfl::ExpTable& et) {
+    const int N = s.N, tid = threadIdx.x;
+    const double beta = s.beta_ex;
+    const double VN = __ldcg(s.V + N);
+    const int off = __ldcg(s.xflags + 4) | __ldcg(s.xflags + 5);
+    const int order = s.Vp ? __ldcg(s.xflags + kExchOrder) : 1;
+    for (int m = tid; m <= N; m += blockDim.x) {
+        const double v = __ldcg(s.V + m), vb = m >= 1 ? __ldcg(s.Vb + m) : 0.0, vh = s.Vh[m];
+        double p = v, pb = vb;
+        bool ext = false;
+        if (s.Vp && extrapolate) {
+            p = s.Vp[m];
+            pb = s.Vp[N + 1 + m];
+            ext = isfinite(p) && isfinite(pb);
+        }
+        if (m >= 1) {
+            s.rowR[m - 1] = exp_df(-beta * (vh + vb - VN), et);
+            s.rowC[m - 1] = exp_df(-beta * (v + vb - VN), et);
+        }
+        s.Vh[m] = ext ? 2.0 * v - p : v;
+        s.Vbh[m] = ext ? 2.0 * vb - pb : vb;
+        if (s.Vp) {
+            s.Vp[m] = v;
+            s.Vp[N + 1 + m] = vb;
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        s.xflags[2] = 0;
+        s.xflags[3] = (off & 2) || ((off & 1) && order);
+        if (s.Vp) s.xflags[kExchOrder] = extrapolate;
+        s.Vb[0] = VN;  // V_backwards[0] = V[N] (:127)
+        s.scal[0] = VN;
+    }
+}
+
 __device__ __noinline__ void band_standalone_tail(const Sys& s, int dir, double* ys, const dfl::ExpTable& etbl,
                                                   int band, bool dense, int* last_band) {
     const int tid = threadIdx.x;
     const int allow_exact = !((volatile int*)s.xflags)[7];  // the estimate was fresh
     int retried = 0;
-    if (solve_direction(s, dir, 0, ys, allow_exact, ys, 0, &etbl)) {
-        if (tid == 0) atomicAdd(&s.xflags[kExchRetryCount], 1);
-        estimate_direction(s, dir, reinterpret_cast<float*>(ys));  // 3 (N+1) floats fit in ys
-        __syncthreads();
-        weights_direction(s, dir, nullptr);  // CUDA's exp (a rare path)
-        __syncthreads();
-        solve_direction(s, dir, 0, ys, 1, nullptr, 1, &etbl);
-        retried = 1;
+    if (finish_direction(s, dir, ys, etbl, last_band)) {
+        if (allow_exact) {
+            solve_direction(s, dir, 0, ys, 1, ys, 0, &etbl);
+        } else {
+            if (tid == 0) atomicAdd(&s.xflags[kExchRetryCount], 1);
+            estimate_direction(s, dir, reinterpret_cast<float*>(ys));  // 3 (N+1) floats fit in ys
+            __syncthreads();
+            weights_direction(s, dir, nullptr);  // CUDA's exp (a rare path)
+            __syncthreads();
+            solve_direction(s, dir, 0, ys, 1, nullptr, 1, &etbl);
+            retried = 1;
+        }
     }
-    __threadfence();
     __syncthreads();
     if (tid == 0) {
+        __threadfence();  // after the block's barrier: its results before the count
         // 1 per direction, 16 per direction that was redone
         const int mine = retried ? 16 : 1;
         const int prev = atomicAdd(&s.xflags[kExchBandCount], mine);
@@ -795,7 +876,7 @@ __device__ __noinline__ void band_standalone_tail(const Sys& s, int dir, double*
     __syncthreads();
     if (*last_band == 0) return;
     __threadfence();
-    solve_finish(s, *last_band != 3 && !allow_exact, &etbl);
+    finish_both(s, *last_band != 3 && !allow_exact, etbl);
     if (tid == 0) {
         s.xflags[6] = 0;
         // full exterior-force rows after a dense solve or a redone direction
@@ -803,6 +884,188 @@ __device__ __noinline__ void band_standalone_tail(const Sys& s, int dir, double*
         s.xflags[kExchBand] = 0;  // the next evaluation's weights measure it anew
         s.xflags[kExchBandCount] = 0;
     }
+}
+
+// The banded solve by FP32 elimination with FP64 residuals (bands up to 32).
+// One warp issues an FP64 instruction every 64 cycles and a dependent
+// multiply-add takes 65 (measured), so the chain over the nodes in FP64 costs
+// 111 cycles a node whatever its arrangement.  Here each 32-node block's
+// unit lower triangle (I - L) is inverted in FP32, all blocks side by side
+// (one warp each: inv = (I - L)^-1 and T = inv U with U the rows' weights on
+// the previous block's last cw >= band nodes), after which a right-hand side
+// is solved by a product with inv per block (side by side) and one cw-term
+// sum per block in sequence, e_b = inv rho_b + T e_{b-1}: about 100 cycles a
+// block of 32 nodes.  y starts at 0 with rho the unit vector; every further
+// round takes the residual rho = W y - y in FP64 (all nodes side by side) and
+// adds the correction to y in FP64, which gains about six digits a round,
+// until the last correction is below 1e-10: three rounds, and the result's
+// error is that of an FP64 residual, as in the substitution.  Gives up (false;
+// block-uniform) where y leaves [1e-20, 1e20], so that corrections of 1e-16
+// still are FP32 numbers, or does not converge.
+// `Ls`: kBandThreads / 32 x 1024 floats; `fs`: 32 nb floats; `store`: nb
+// blocks of T [32][cw + 1] and inv [32][36].
+constexpr int kBandWarps = kBandThreads / 32;
+constexpr int kBandRefined = 32;    // the band it takes
+// Blocks from which it is the faster form: its code is long and runs once, so
+// few blocks pay more for fetching it than they save (steps of N = 256, 9
+// blocks, and N = 1024, 33 blocks, 2-3% slower with it; N = 4096, 129 blocks,
+// 8.21 -> 7.82 ms for 4 steps).
+constexpr int kBandRefinedMin = 64;
+constexpr int kBandStore = 32 * 33 + 32 * 36;  // floats per block at most (behind ysol)
+// A double rounded to float by bit patterns, 0 below 2^-126 and infinite above
+// a float's range (the conversion instruction takes the FP64 pipe for 128
+// cycles a warp).
+__device__ __forceinline__ float f32_of(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), e = (hi >> 20) & 0x7ffu;
+    unsigned q = ((e - 896u) << 23 | (hi & 0xfffffu) << 3 | lo >> 29) + ((lo >> 28) & 1u);
+    if (e <= 896u) q = 0u;
+    if (e >= 1151u) q = 0x7f800000u | (e == 0x7ffu ? (hi & 0xfffffu) | lo : 0u);
+    return __uint_as_float(q | (hi & 0x80000000u));
+}
+// e_b = inv rho_b + T e_{b-1} over the blocks, by one warp (lane = row): fs
+// holds inv rho_b and receives e_b.  The next block's T is loaded, and the one
+// six blocks on prefetched, while this one is summed.
+template <int CW>
+__device__ __forceinline__ void band_sequence(int nb, float* fs, const float* store, int lane) {
+    constexpr int ldt = CW + 1, per = 32 * ldt + 32 * 36;
+    float e = fs[lane], next[CW];
+    auto fetch = [&](int b) {
+#pragma unroll
+        for (int c = 0; c < CW; ++c) next[c] = store[(size_t)b * per + lane * ldt + c];
+    };
+    fetch(1);
+    for (int b = 1; b < nb; ++b) {
+        float T[CW], s[4] = {fs[32 * b + lane], 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int c = 0; c < CW; ++c) T[c] = next[c];
+        if (b + 6 < nb)
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(store + (size_t)(b + 6) * per + lane * ldt));
+        if (b + 1 < nb) fetch(b + 1);
+#pragma unroll
+        for (int c = 0; c < CW; ++c) s[c & 3] = fmaf(T[c], __shfl_sync(0xffffffffu, e, 32 - CW + c), s[c & 3]);
+        e = (s[0] + s[1]) + (s[2] + s[3]);
+        fs[32 * b + lane] = e;
+    }
+}
+__device__ __noinline__ bool band_refined(const double* __restrict__ W, int nn, int band, double* ys, float* fs,
+                                          float* Ls, float* store) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nb = (nn + 31) / 32, cw = (band + 7) & ~7, ldt = cw + 1, per = 32 * ldt + 32 * 36;
+    for (int b = warp; b < nb; b += kBandWarps) {
+        float* L = Ls + warp * 1024;
+        float T[32], I[32];
+        // row r's weights on the 32 nodes before it, one load a row; those of
+        // this block go to L, those of the previous block to the lane of
+        // their column
+#pragma unroll
+        for (int r0 = 0; r0 < 32; r0 += 16) {
+            double w[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                const int m = 32 * b + r0 + q, c = m - 32 + lane;
+                w[q] = m < nn && c >= 0 && lane >= 32 - band ? W[tri(m - 1) + c] : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                const int r = r0 + q;
+                const float v = f32_of(w[q]);
+                const float t = __shfl_sync(0xffffffffu, v, (lane - r) & 31);
+                T[r] = lane >= r ? t : 0.0f;
+                if (lane + r >= 32) L[r * 32 + lane + r - 32] = v;
+            }
+        }
+        __syncwarp();
+        // rows in order; lane = column (of the previous block for T, of this one for inv)
+#pragma unroll
+        for (int r = 0; r < 32; ++r) {
+            float t[4] = {T[r], 0.0f, 0.0f, 0.0f}, i[4] = {lane == r ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int q = 0; q < r; q += 4) {
+                const float4 l = *reinterpret_cast<const float4*>(L + r * 32 + q);  // columns below r are used
+                t[0] = fmaf(l.x, T[q], t[0]);
+                i[0] = fmaf(l.x, I[q], i[0]);
+                if (q + 1 < r) {
+                    t[1] = fmaf(l.y, T[q + 1], t[1]);
+                    i[1] = fmaf(l.y, I[q + 1], i[1]);
+                }
+                if (q + 2 < r) {
+                    t[2] = fmaf(l.z, T[q + 2], t[2]);
+                    i[2] = fmaf(l.z, I[q + 2], i[2]);
+                }
+                if (q + 3 < r) {
+                    t[3] = fmaf(l.w, T[q + 3], t[3]);
+                    i[3] = fmaf(l.w, I[q + 3], i[3]);
+                }
+            }
+            T[r] = (t[0] + t[1]) + (t[2] + t[3]);
+            I[r] = (i[0] + i[1]) + (i[2] + i[3]);
+        }
+        float* st = store + (size_t)b * per;
+#pragma unroll
+        for (int r = 0; r < 32; ++r) {
+            if (lane >= 32 - cw) st[r * ldt + lane - (32 - cw)] = T[r];
+            st[32 * ldt + r * 36 + lane] = I[r];
+        }
+        __syncwarp();  // the next block overwrites L
+    }
+    for (int m = tid; m < nn; m += kBandThreads) ys[m] = 0.0;
+    __syncthreads();
+    for (int round = 0; round < 6; ++round) {
+        for (int m = tid; m < 32 * nb; m += kBandThreads) {
+            double r = m == 0 ? 1.0 : 0.0;
+            if (round > 0 && m < nn) {
+                const double* row = W + (m >= 1 ? tri(m - 1) : 0);
+                double r1 = -ys[m];
+                int c = max(0, m - band);
+                if ((m - c) & 1) {
+                    r = fma(row[c], ys[c], r);
+                    ++c;
+                }
+#pragma unroll 8
+                for (; c < m; c += 2) {
+                    r = fma(row[c], ys[c], r);
+                    r1 = fma(row[c + 1], ys[c + 1], r1);
+                }
+                r += r1;
+            }
+            fs[m] = f32_of(r);
+        }
+        __syncthreads();
+        for (int b = warp; b < nb; b += kBandWarps) {
+            const float4* inv = reinterpret_cast<const float4*>(store + (size_t)b * per + 32 * ldt + lane * 36);
+            const float rho = fs[32 * b + lane];
+            float z[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+                const float4 v = inv[t];
+                z[0] = fmaf(v.x, __shfl_sync(0xffffffffu, rho, 4 * t), z[0]);
+                z[1] = fmaf(v.y, __shfl_sync(0xffffffffu, rho, 4 * t + 1), z[1]);
+                z[2] = fmaf(v.z, __shfl_sync(0xffffffffu, rho, 4 * t + 2), z[2]);
+                z[3] = fmaf(v.w, __shfl_sync(0xffffffffu, rho, 4 * t + 3), z[3]);
+            }
+            fs[32 * b + lane] = (z[0] + z[1]) + (z[2] + z[3]);
+        }
+        __syncthreads();
+        if (warp == 0) {
+            if (cw == 8) band_sequence<8>(nb, fs, store, lane);
+            else if (cw == 16) band_sequence<16>(nb, fs, store, lane);
+            else if (cw == 24) band_sequence<24>(nb, fs, store, lane);
+            else band_sequence<32>(nb, fs, store, lane);
+        }
+        __syncthreads();
+        int more = 0, bad = 0;
+        for (int m = tid; m < nn; m += kBandThreads) {
+            const float e = fs[m];
+            const double y = ys[m] + f32_to_f64(e);
+            const float yf = fabsf(f32_of(y));
+            ys[m] = y;
+            if (!(fabsf(e) <= 1e-10f * yf)) more = 1;
+            if (!(yf >= 1e-20f && yf <= 1e20f)) bad = 1;
+        }
+        if (__syncthreads_or(bad)) return false;
+        if (!__syncthreads_or(more)) return true;
+    }
+    return false;
 }
 
 __global__ void __launch_bounds__(kBandThreads) k_exch_solve_band(Sys s, int phase, double* ysol, int standalone) {
@@ -820,10 +1083,29 @@ __global__ void __launch_bounds__(kBandThreads) k_exch_solve_band(Sys s, int pha
     double* y = ysol + (size_t)dir * (s.N + 1);
     const int nnpad = (nn + 1) & ~1;
     double* ys = bsm;                    // [nn]
-    double* wdiag = bsm + nnpad;         // [2][32][32]: block b's diagonal block, row-major
-    double* wfold = wdiag + 2 * 1024;    // [2][32][64]: block b's rows, columns 32b - 64 .. 32b - 1
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nb = (nn + 31) / 32;
+    const int nb = (nn + 31) / 32, nbmax = (s.N + 1 + 31) / 32;
+    float* fs = reinterpret_cast<float*>(bsm + nnpad);       // [32 nb]
+    float* Ls = fs + 32 * nbmax;                             // band_refined's rows
+    double* wdiag = reinterpret_cast<double*>(Ls);  // [2][32][32]: block b's diagonal block, row-major
+    double* wfold = wdiag + 2 * 1024;    // [2][32][64]: block b's rows, columns 32b - 64 .. 32b - 1
+    // the exponential's table beside the first loads (used after barriers)
+    if (tid >= kBandThreads - 256) {
+        const int j = tid - (kBandThreads - 256);
+        float h, l;
+        split_f32(kExp2Table256[j], h, l);
+        const dfl::df n = dfl::fast_two_sum(h, l);
+        etbl.hi[j] = n.hi;
+        etbl.lo[j] = n.lo;
+    }
+    bool solved = false;
+    if (band <= kBandRefined && nb >= kBandRefinedMin) {
+        float* store = reinterpret_cast<float*>(ysol + 2 * ((size_t)s.N + 1)) + (size_t)dir * nbmax * kBandStore;
+        solved = band_refined(W, nn, band, ys, fs, Ls, store);
+        if (solved)
+            for (int m = tid; m < nn; m += blockDim.x) y[m] = ys[m];
+        __syncthreads();
+    }
     // Threads t0.. stage block b's weights: row r of the block needs columns
     // 32b - 64 .. 32b + r - 1 of its packed row (contiguous), taken as one
     // row-major index e = 96 r + q (q < 64: fold, else diagonal) so that a
@@ -857,11 +1139,11 @@ __global__ void __launch_bounds__(kBandThreads) k_exch_solve_band(Sys s, int pha
         for (int m = tid; m < nn; m += blockDim.x) y[m] = ys[m];
         __syncthreads();
     }
-    if (!dense) stage(0, 0, blockDim.x);
+    if (!dense && !solved) stage(0, 0, blockDim.x);
     __syncthreads();
-    const int i = tid >> 3, part = tid & 7;  // fold role: row of the block, 8 of its 64 columns
+    const int i = tid >> 3, part = tid & 7;  // fold role (threads below 256): row of the block, 8 of its 64 columns
     const int dband = dense ? 32 : band;  // the diagonal chain's reach
-    for (int b = 0; b < (dense ? 0 : nb); ++b) {
+    for (int b = 0; b < (dense || solved ? 0 : nb); ++b) {
         const double* f = wfold + (b & 1) * 2048;
         double sum = 0.0;
         // columns more than `band` before the block's first row hold exact
@@ -869,12 +1151,12 @@ __global__ void __launch_bounds__(kBandThreads) k_exch_solve_band(Sys s, int pha
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const int col = 8 * part + q, c = 32 * b - 64 + col;
-            if (c >= 0 && col >= 64 - band) sum = fma(f[i * 64 + col], ys[c], sum);
+            if (i < 32 && c >= 0 && col >= 64 - band) sum = fma(f[i * 64 + col], ys[c], sum);
         }
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
         sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-        if (part == 0) accb[i] = sum;
+        if (part == 0 && i < 32) accb[i] = sum;
         __syncthreads();
         if (warp == 0) {
             const double* d = wdiag + (b & 1) * 1024;
@@ -902,16 +1184,13 @@ __global__ void __launch_bounds__(kBandThreads) k_exch_solve_band(Sys s, int pha
     // CTA that finishes second runs solve_finish when both directions
     // succeeded and marks the evaluation done.
     if (phase != 0) return;
-    fill_exp_table_df(etbl);
-    __syncthreads();
     if (standalone) {
         band_standalone_tail(s, dir, ys, etbl, band, dense, &last_band);
         return;
     }
-    const int gave_up = solve_direction(s, dir, 0, ys, 0, ys, 0, &etbl);
-    __threadfence();
-    __syncthreads();
+    const int gave_up = finish_direction(s, dir, ys, etbl, &last_band);
     if (tid == 0) {
+        __threadfence();  // after the block's barrier: its results before the count
         // count 2 per direction that succeeded, 1 per direction that gave up
         const int prev = atomicAdd(&s.xflags[kExchBandCount], gave_up ? 1 : 2);
         last_band = prev > 0 ? (prev + (gave_up ? 1 : 2)) : 0;
@@ -920,7 +1199,7 @@ __global__ void __launch_bounds__(kBandThreads) k_exch_solve_band(Sys s, int pha
     if (last_band == 0) return;
     __threadfence();
     if (last_band == 4) {
-        solve_finish(s, ((volatile int*)s.xflags)[7], &etbl);
+        finish_both(s, ((volatile int*)s.xflags)[7], etbl);
         if (tid == 0) {
             s.xflags[kExchBandLast] = s.xflags[kExchBand];
             s.xflags[kExchBand] = 0;  // the next evaluation's weights measure it anew
@@ -932,8 +1211,16 @@ __global__ void __launch_bounds__(kBandThreads) k_exch_solve_band(Sys s, int pha
 
 bool banded_solve_fits(const Sys& s) { return s.N + 1 <= kBandMaxN; }
 
+static int band_blocks(const Sys& s) { return (s.N + 1 + 31) / 32; }
+// Floats of band_refined's store behind ysol (both directions).
+static size_t band_store_floats(const Sys& s) {
+    return band_blocks(s) < kBandRefinedMin || !banded_solve_fits(s) ? 0 : 2 * (size_t)band_blocks(s) * kBandStore;
+}
 size_t banded_solve_smem(const Sys& s) {
-    return sizeof(double) * ((((size_t)s.N + 2) & ~(size_t)1) + 2 * 1024 + 2 * 2048);
+    const size_t fp64 = sizeof(double) * (2 * 1024 + 2 * 2048);
+    const size_t refined = band_blocks(s) < kBandRefinedMin ? 0 : sizeof(float) * kBandWarps * 1024;
+    return sizeof(double) * (((size_t)s.N + 2) & ~(size_t)1) + sizeof(float) * 32 * (size_t)band_blocks(s) +
+           std::max(refined, fp64);
 }
 
 
@@ -1068,8 +1355,9 @@ int launch_exchange_energies(const Sys& s, int D, cudaStream_t st, double* work)
 }
 
 // y of both directions for the banded solve and the multi-SM solve (and g
-// for the multi-SM estimate before them); publication flags for the latter.
-size_t exchange_grid_doubles(const Sys& s) { return 2 * ((size_t)s.N + 1); }
+// for the multi-SM estimate before them), then the banded solve's store;
+// publication flags for the multi-SM kernels.
+size_t exchange_grid_doubles(const Sys& s) { return 2 * ((size_t)s.N + 1) + (band_store_floats(s) + 1) / 2; }
 size_t exchange_grid_flags(const Sys& s) {
     return s.N >= kFlatEnergiesMinN ? 2 * (((size_t)s.N + 1 + 31) / 32) + 1 : 1;
 }
