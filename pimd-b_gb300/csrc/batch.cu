@@ -67,6 +67,51 @@ struct BatchRep {
 };
 
 constexpr int kBatchMaxThreads = 512;
+
+// The threads that run one replica's step: one CTA, or (kCl) the CTAs of a
+// thread-block cluster.  With fewer replicas than the GPU holds CTAs the step's
+// time is the largest replica's on one SM (its FP64 pipe), so the beads, the
+// element passes and the exchange's rows are spread over the cluster's SMs and
+// the two directions of the exchange run on two of them.  sync() orders the
+// team's global memory too (the cluster barrier's release and acquire).
+template <bool kCl>
+struct Team {
+    static __device__ __forceinline__ int rank() {
+        if constexpr (!kCl) return 0;
+        unsigned r;
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+        return (int)r;
+    }
+    static __device__ __forceinline__ int size() {
+        if constexpr (!kCl) return 1;
+        unsigned r;
+        asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+        return (int)r;
+    }
+    static __device__ __forceinline__ int tid() { return kCl ? rank() * (int)blockDim.x + (int)threadIdx.x : (int)threadIdx.x; }
+    static __device__ __forceinline__ int threads() { return kCl ? size() * (int)blockDim.x : (int)blockDim.x; }
+    static __device__ __forceinline__ int warp() { return tid() >> 5; }
+    static __device__ __forceinline__ int warps() { return threads() >> 5; }
+    static __device__ __forceinline__ void sync() {
+        if constexpr (kCl)
+            asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        else
+            __syncthreads();
+    }
+    // a double of CTA r's shared memory, at this CTA's address `p` of it
+    static __device__ __forceinline__ double peer(const double* p, int r) {
+        unsigned a = (unsigned)__cvta_generic_to_shared(p), q;
+        double v;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(q) : "r"(a), "r"(r));
+        asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(q) : "memory");
+        return v;
+    }
+    static __device__ __forceinline__ void set_peer(int* p, int r, int v) {
+        unsigned a = (unsigned)__cvta_generic_to_shared(p), q;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(q) : "r"(a), "r"(r));
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(q), "r"(v) : "memory");
+    }
+};
 // Beads of a replica with normal modes: each warp holds 8 P doubles of one
 // particle pair's lines in shared memory.
 constexpr int kBatchMaxNmBeads = 256;
@@ -81,10 +126,12 @@ __device__ __forceinline__ void normal_pair(const Sys& s, long long step, int su
     z1 = f32_to_f64(z.y);
 }
 
-// Sums v[0..D) over the block; every thread receives the totals.  `sh`
-// holds 3 * 32 doubles.
-template <int D>
-__device__ __forceinline__ void block_sum_axes(double* v, double* sh) {
+// Sums v[0..D) over the team; every thread receives the totals.  `sh` holds
+// 3 * 32 doubles; a cluster adds its CTAs' totals in rank order from `com`
+// (two slots of 4 doubles used in turn, `turn`: a slot is written again only
+// after the barrier of the sum in between).
+template <int D, bool kCl>
+__device__ __forceinline__ void block_sum_axes(double* v, double* sh, double (*com)[4], int& turn) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
     for (int a = 0; a < D; ++a) {
@@ -97,6 +144,20 @@ __device__ __forceinline__ void block_sum_axes(double* v, double* sh) {
         double t = 0.0;
         for (int k = 0; k < nw; ++k) t += sh[a * 32 + k];
         v[a] = t;
+    }
+    if constexpr (kCl) {
+        double* slot = com[turn & 1];
+        ++turn;
+        if (threadIdx.x == 0)
+#pragma unroll
+            for (int a = 0; a < D; ++a) slot[a] = v[a];
+        Team<true>::sync();
+#pragma unroll
+        for (int a = 0; a < D; ++a) {
+            double t = 0.0;
+            for (int r = 0; r < Team<true>::size(); ++r) t += Team<true>::peer(slot + a, r);
+            v[a] = t;
+        }
     }
     __syncthreads();
 }
@@ -142,11 +203,11 @@ __device__ __forceinline__ double2 nm_kick_pair(const Sys& s, int b, int a, int 
 // them latency-bound.  The elements are taken in the same per-thread order
 // as one pair at a time (the same sums, bit for bit).
 constexpr int kPassUnroll = 4;
-template <int D, typename R>
+template <int D, typename R, bool kCl>
 __device__ __forceinline__ void momenta_pass(const Sys& s, long long step, int substep, const double* cm, bool com_in,
                                              bool kick, bool o, bool drift, double* sum, bool nmkick = false) {
     const int N = s.N, H = (N + 1) / 2;
-    const int total = s.P * H, stride = blockDim.x;
+    const int total = s.P * H, stride = Team<kCl>::threads();
     // loop constants kept in registers (opaque: not recomputed per element)
     double hdt = 0.5 * s.dt, c1 = s.c1, c2 = s.c2, dt_m = s.dt_m;
     asm volatile("" : "+d"(hdt), "+d"(c1), "+d"(c2), "+d"(dt_m));
@@ -154,7 +215,7 @@ __device__ __forceinline__ void momenta_pass(const Sys& s, long long step, int s
     for (int a = 0; a < D; ++a) {
         double sa = 0.0;
         const double cma = com_in ? cm[a] : 0.0;
-        for (int q0 = threadIdx.x; q0 < total; q0 += kPassUnroll * stride) {
+        for (int q0 = Team<kCl>::tid(); q0 < total; q0 += kPassUnroll * stride) {
             double2 pv[kPassUnroll], fv[kPassUnroll], xv[kPassUnroll];
 #pragma unroll
             for (int k = 0; k < kPassUnroll; ++k) {
@@ -541,9 +602,9 @@ __host__ __device__ constexpr size_t xforces_f32_floats(int D, int N) { return 4
 // floats, each lane's terms and the warp's lanes summed with two-sum error
 // terms.  Lanes 0..D-1 add the interior neighbour spring and write axis
 // a = lane: one FP64 add per row joins the result to f.
-template <int D>
+template <int D, bool kCl>
 __device__ void batch_exchange_forces_f32(const Sys& s, float* sm) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = Team<kCl>::warp(), nw = Team<kCl>::warps();
     const int N = s.N, P = s.P;
     float* xh = sm;  // (side D + a) N + i; side 0 bead 1, 1 bead P
     float* xl = xh + 2 * D * N;
@@ -733,10 +794,13 @@ __device__ inline void batch_estimate(const Sys& s, int dir, float* fsm) {
 // The Feldman-Hirshberg exchange of one replica by the whole block; adds the
 // exterior springs to f on beads 1 and P (which hold the physical forces).
 // R = float: weights and exterior forces on the FP32 pipe (above).
-template <int D, typename R>
+template <int D, typename R, bool kCl>
 __device__ void batch_exchange(const Sys& s, unsigned char* work, const double* tbl, const dfl::ExpTable* etbl) {
     constexpr bool kMixed = sizeof(R) == 4;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    using T = Team<kCl>;
+    const int lane = threadIdx.x & 31, warp = T::warp(), nw = T::warps();
+    // a cluster's first two CTAs take a direction each
+    const bool fwd = !kCl || T::rank() == 0, bwd = !kCl || T::rank() == 1;
     const int N = s.N;
     // the interior links |x1_{u+1} - xP_u|^2 once per u (shared memory),
     // instead of once per cycle-energy entry
@@ -744,43 +808,44 @@ __device__ void batch_exchange(const Sys& s, unsigned char* work, const double* 
     for (int u = threadIdx.x; u < N - 1; u += blockDim.x) link[u] = sepsq<D>(s, s.P - 1, u, 0, u + 1);
     __syncthreads();
     for (int v = warp; v < N; v += nw) energy_row<D>(s, v, lane, link);
-    __syncthreads();
+    T::sync();
     int fresh = ((volatile int*)s.xflags)[3];
-    __syncthreads();
+    T::sync();
     for (int attempt = 0; attempt < 2; ++attempt) {
         if (fresh) {
-            batch_estimate(s, 0, reinterpret_cast<float*>(work));
-            __syncthreads();
-            batch_estimate(s, 1, reinterpret_cast<float*>(work));
-            __syncthreads();
+            if (fwd) batch_estimate(s, 0, reinterpret_cast<float*>(work));
+            if constexpr (!kCl) __syncthreads();
+            if (bwd) batch_estimate(s, 1, reinterpret_cast<float*>(work));
+            T::sync();
         }
         if (kMixed) {
-            weights_df_block(s, *etbl, reinterpret_cast<float*>(work));
+            weights_df_block(s, *etbl, reinterpret_cast<float*>(work), warp, nw);
         } else {
             for (int p = warp; p < N; p += nw) {
                 const double inv = recip_row(p);
                 for (int u = lane; u <= p; u += 32) exch_weight(s, p, u, inv, tbl);
             }
         }
-        __syncthreads();
+        T::sync();
         // a reused estimate that fails is replaced by a fresh one (second
         // attempt) rather than by the exact recursion
-        solve_direction(s, 0, 0, reinterpret_cast<double*>(work), fresh, nullptr, 1, etbl);
-        __syncthreads();
-        solve_direction(s, 1, 0, reinterpret_cast<double*>(work), fresh, nullptr, 1, etbl);
-        __syncthreads();
+        if (fwd) solve_direction(s, 0, 0, reinterpret_cast<double*>(work), fresh, nullptr, 1, etbl);
+        if constexpr (!kCl) __syncthreads();
+        if (bwd) solve_direction(s, 1, 0, reinterpret_cast<double*>(work), fresh, nullptr, 1, etbl);
+        T::sync();
         const int retry = ((volatile int*)s.xflags)[6];
-        __syncthreads();
+        T::sync();
         if (!retry) break;
-        if (threadIdx.x == 0) s.xflags[6] = 0;
+        if (fwd && threadIdx.x == 0) s.xflags[6] = 0;
         fresh = 1;
-        __syncthreads();
+        T::sync();
     }
-    solve_finish(s, 0, etbl);
+    if (fwd) solve_finish(s, 0, etbl);
+    if constexpr (kCl) T::sync();
     // the exact fallback's probabilities come from their exponentials: FP64 rows
     if (kMixed && !((volatile int*)s.xflags)[0]) {
         __syncthreads();
-        batch_exchange_forces_f32<D>(s, reinterpret_cast<float*>(work));
+        batch_exchange_forces_f32<D, kCl>(s, reinterpret_cast<float*>(work));
         return;
     }
     // beads 1 and P staged in the (now free) shared scratch for the forces
@@ -803,11 +868,11 @@ __device__ void batch_exchange(const Sys& s, unsigned char* work, const double* 
 
 // [COM], half-kick with the normal-mode kick force, Cartesian -> modes, the
 // exact free ring-polymer rotation, modes -> Cartesian; x and p written.
-template <int D>
+template <int D, bool kCl>
 __device__ __noinline__ void nm_propagate_block(const Sys& s, const NmTabs& nm, const double* cm, bool com_in, double* wsm) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = Team<kCl>::warp(), nw = Team<kCl>::warps();
     const int P = s.P, N = s.N, H = (N + 1) / 2;
-    double* w = wsm + (size_t)warp * 8 * P;  // x0 x1 p0 p1 | q0 q1 u0 u1
+    double* w = wsm + (size_t)(threadIdx.x >> 5) * 8 * P;  // x0 x1 p0 p1 | q0 q1 u0 u1
     const double hdt = 0.5 * s.dt;
     for (int line = warp; line < D * H; line += nw) {
         const int a = line / H, i0 = 2 * (line - a * H);
@@ -882,12 +947,12 @@ __device__ __noinline__ void nm_propagate_block(const Sys& s, const NmTabs& nm, 
 // mode k drawn as the Cartesian ones of bead k: pair index (k D + a)
 // ceil(N/2) + i/2); p written, and its per-axis sums (this thread's share)
 // in `sum`.
-template <int D, typename R>
+template <int D, typename R, bool kCl>
 __device__ __noinline__ void nm_thermo_block(const Sys& s, const NmTabs& nm, long long step, int substep, const double* cm,
                                 bool com_in, double* sum, double* wsm) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = Team<kCl>::warp(), nw = Team<kCl>::warps();
     const int P = s.P, N = s.N, H = (N + 1) / 2;
-    double* w = wsm + (size_t)warp * 8 * P;  // p0 p1 | u0 u1
+    double* w = wsm + (size_t)(threadIdx.x >> 5) * 8 * P;  // p0 p1 | u0 u1
     for (int a = 0; a < D; ++a) sum[a] = 0.0;
     for (int line = warp; line < D * H; line += nw) {
         const int a = line / H, i2 = line - a * H, i0 = 2 * i2;
@@ -934,10 +999,12 @@ __device__ __noinline__ void nm_thermo_block(const Sys& s, const NmTabs& nm, lon
     }
 }
 
-template <int D, typename R>
+template <int D, typename R, bool kCl>
 __device__ void batch_replica(const Sys& s, int flags, const NmTabs& nm, long long step, int mode, double* red,
-                              unsigned char* work, const double* tbl, const dfl::ExpTable* etbl) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+                              unsigned char* work, const double* tbl, const dfl::ExpTable* etbl, double (*com)[4],
+                              int& turn) {
+    using T = Team<kCl>;
+    const int lane = threadIdx.x & 31, warp = T::warp(), nw = T::warps();
     const bool langevin = flags & BF_LANGEVIN, fixcom = flags & BF_FIXCOM;
     const bool nmprop = flags & BF_NM, nmthermo = langevin && (flags & BF_NMTHERMO);
     const bool cart_langevin = langevin && !nmthermo;
@@ -949,62 +1016,62 @@ __device__ void batch_replica(const Sys& s, int flags, const NmTabs& nm, long lo
     if (mode & BM_HEAD) {
         // O-step (substep 0) and the sums for the COM removal
         if (nmthermo || cart_langevin || fixcom) {
-            if (nmthermo) nm_thermo_block<D, R>(s, nm, step, 0, cm, false, sum, wsm);
-            else momenta_pass<D, R>(s, step, 0, cm, false, false, cart_langevin, false, sum);
+            if (nmthermo) nm_thermo_block<D, R, kCl>(s, nm, step, 0, cm, false, sum, wsm);
+            else momenta_pass<D, R, kCl>(s, step, 0, cm, false, false, cart_langevin, false, sum);
             if (fixcom) {
-                block_sum_axes<D>(sum, red);
+                block_sum_axes<D, kCl>(sum, red, com, turn);
 #pragma unroll
                 for (int a = 0; a < D; ++a) cm[a] = sum[a] * inv_np;
             } else {
-                __syncthreads();
+                T::sync();
             }
         }
         // [COM], B, A (velocity_verlet.cpp:9-12) or the normal-mode
         // propagation up to the forces (normal_modes_propagator.cpp:19-63)
-        if (nmprop) nm_propagate_block<D>(s, nm, cm, fixcom, wsm);
-        else momenta_pass<D, R>(s, step, 0, cm, fixcom, true, false, true, sum);
-        __syncthreads();
+        if (nmprop) nm_propagate_block<D, kCl>(s, nm, cm, fixcom, wsm);
+        else momenta_pass<D, R, kCl>(s, step, 0, cm, fixcom, true, false, true, sum);
+        T::sync();
     }
     if (mode & BM_FORCES) {
-        unsigned char* stage = work + (size_t)warp * stage_bytes<D>() * s.N;
+        unsigned char* stage = work + (size_t)(threadIdx.x >> 5) * stage_bytes<D>() * s.N;
         for (int b = warp; b < s.P; b += nw) bead_forces_warp<D, R>(s, b, lane, stage);
-        __syncthreads();
+        T::sync();
         if (s.bosonic) {
-            batch_exchange<D, R>(s, work, tbl, etbl);
-            __syncthreads();
+            batch_exchange<D, R, kCl>(s, work, tbl, etbl);
+            T::sync();
         }
     }
     if (mode & BM_TAIL) {
         // B (the normal-mode kick force under the normal-mode propagator),
         // O-step (substep 1), COM removal
         if (nmthermo) {
-            if (nmprop) momenta_pass<D, R>(s, step, 1, cm, false, true, false, false, sum, true);
-            else momenta_pass<D, R>(s, step, 1, cm, false, true, false, false, sum, false);
-            __syncthreads();
-            nm_thermo_block<D, R>(s, nm, step, 1, cm, false, sum, wsm);
+            if (nmprop) momenta_pass<D, R, kCl>(s, step, 1, cm, false, true, false, false, sum, true);
+            else momenta_pass<D, R, kCl>(s, step, 1, cm, false, true, false, false, sum, false);
+            T::sync();
+            nm_thermo_block<D, R, kCl>(s, nm, step, 1, cm, false, sum, wsm);
         } else if (nmprop) {
-            momenta_pass<D, R>(s, step, 1, cm, false, true, cart_langevin, false, sum, true);
+            momenta_pass<D, R, kCl>(s, step, 1, cm, false, true, cart_langevin, false, sum, true);
         } else {
-            momenta_pass<D, R>(s, step, 1, cm, false, true, cart_langevin, false, sum, false);
+            momenta_pass<D, R, kCl>(s, step, 1, cm, false, true, cart_langevin, false, sum, false);
         }
         if (fixcom) {
-            block_sum_axes<D>(sum, red);
+            block_sum_axes<D, kCl>(sum, red, com, turn);
 #pragma unroll
             for (int a = 0; a < D; ++a) cm[a] = sum[a] * inv_np;
-            momenta_pass<D, R>(s, step, 1, cm, true, false, false, false, sum);
+            momenta_pass<D, R, kCl>(s, step, 1, cm, true, false, false, false, sum);
         }
-        __syncthreads();
+        T::sync();
     }
     if (mode & BM_ESTIMATORS) {
-        if (s.bosonic) estimators_block(s, s.P, reinterpret_cast<double*>(work));
-        __syncthreads();
+        if (s.bosonic && T::rank() == 0) estimators_block(s, s.P, reinterpret_cast<double*>(work));
+        T::sync();
     }
 }
 
 // One launch: every replica through `mode`.  ctl[0] is the work counter,
 // ctl[1] counts finished CTAs; the last CTA resets both and, with
 // BM_ADVANCE, advances the step counter.
-template <int D, typename R>
+template <int D, typename R, bool kCl>
 __global__ void __launch_bounds__(kBatchMaxThreads)
     k_batch(const BatchRep* __restrict__ reps, const int* __restrict__ order, int nrep, int* ctl,
             long long* step_ctr, int mode) {
@@ -1014,14 +1081,23 @@ __global__ void __launch_bounds__(kBatchMaxThreads)
     __shared__ Sys ss;
     __shared__ NmTabs snm;
     __shared__ int item, sflags;
+    __shared__ double com[2][4];  // a cluster's centre-of-mass sums
+    using T = Team<kCl>;
+    int turn = 0;
     __shared__ double tbl[32];  // exp_tang's table
     __shared__ dfl::ExpTable etbl;  // 2^(j/256) as double-floats (bit patterns)
     if (threadIdx.x < 32) tbl[threadIdx.x] = kExp2Table[threadIdx.x];
     fill_exp_table_df(etbl);
     const long long step = *(volatile long long*)step_ctr;
     for (;;) {
-        if (threadIdx.x == 0) item = atomicAdd(&ctl[0], 1);
-        __syncthreads();
+        if (T::tid() == 0) {
+            const int next = atomicAdd(&ctl[0], 1);
+            if constexpr (kCl)
+                for (int r = 0; r < T::size(); ++r) T::set_peer(&item, r, next);
+            else
+                item = next;
+        }
+        T::sync();
         const int k = item;
         if (k < nrep && threadIdx.x == 0) {
             ss = reps[order[k]].s;
@@ -1030,8 +1106,8 @@ __global__ void __launch_bounds__(kBatchMaxThreads)
         }
         __syncthreads();
         if (k >= nrep) break;
-        batch_replica<D, R>(ss, sflags, snm, step, mode, red, work, tbl, &etbl);
-        __syncthreads();
+        batch_replica<D, R, kCl>(ss, sflags, snm, step, mode, red, work, tbl, &etbl, com, turn);
+        T::sync();
     }
     if (threadIdx.x == 0) {
         __threadfence();
@@ -1094,6 +1170,7 @@ __global__ void k_batch_reset(const BatchRep* __restrict__ reps, int D) {
 using namespace pimdb;
 
 // --------------------------------------------------------------------- host
+constexpr int kBatchMaxCluster = 8;  // the portable size
 struct pimdb_batch {
     int nrep = 0, D = 3, mixed = 0;
     std::vector<pimdb_config> cfgs;
@@ -1114,6 +1191,7 @@ struct pimdb_batch {
     double* d_stage = nullptr;  // host-layout staging (htotal doubles)
     cudaStream_t stream = nullptr;
     bool own_stream = false;
+    int cluster = 1;  // CTAs per replica
     int threads = 256, ctas_per_sm = 2, grid = 1, maxN = 1, sms = 1, maxPnm = 0;
     size_t smem = 0;
     bool use_graph = true;
@@ -1152,17 +1230,36 @@ static size_t batch_smem(int D, int maxN, int threads, int maxPnm) {
                     std::max(std::max(xforces, xforces32), nmlines));
 }
 
-template <typename F>
-static void with_kernel(int D, int mixed, F&& f) {
+template <bool kCl, typename F>
+static void with_kernel_of(int D, int mixed, F&& f) {
     if (mixed) {
-        if (D == 1) f(k_batch<1, float>);
-        else if (D == 2) f(k_batch<2, float>);
-        else f(k_batch<3, float>);
+        if (D == 1) f(k_batch<1, float, kCl>);
+        else if (D == 2) f(k_batch<2, float, kCl>);
+        else f(k_batch<3, float, kCl>);
     } else {
-        if (D == 1) f(k_batch<1, double>);
-        else if (D == 2) f(k_batch<2, double>);
-        else f(k_batch<3, double>);
+        if (D == 1) f(k_batch<1, double, kCl>);
+        else if (D == 2) f(k_batch<2, double, kCl>);
+        else f(k_batch<3, double, kCl>);
     }
+}
+template <typename F>
+static void with_kernel(int D, int mixed, bool cluster, F&& f) {
+    if (cluster) with_kernel_of<true>(D, mixed, f);
+    else with_kernel_of<false>(D, mixed, f);
+}
+// A launch of `cluster` CTAs per replica.
+static void batch_config(cudaLaunchConfig_t& c, cudaLaunchAttribute& at, int grid, int threads, size_t smem, int cluster,
+                         cudaStream_t st) {
+    c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = cluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
 }
 
 static int configure_launch(pimdb_batch* b, int threads, int ctas_per_sm) {
@@ -1175,7 +1272,7 @@ static int configure_launch(pimdb_batch* b, int threads, int ctas_per_sm) {
     size_t stat = 0;
     if (cudaGetDevice(&dev) == cudaSuccess)
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    with_kernel(b->D, b->mixed, [&](auto k) {
+    with_kernel(b->D, b->mixed, true, [&](auto k) {
         cudaFuncAttributes fa{};
         if (cudaFuncGetAttributes(&fa, k) == cudaSuccess) stat = fa.sharedSizeBytes;
     });
@@ -1184,10 +1281,13 @@ static int configure_launch(pimdb_batch* b, int threads, int ctas_per_sm) {
         return bfail(b, PIMDB_ERR_CONFIG, "the batched kernel needs " + std::to_string(smem + stat) +
                                               " bytes of shared memory for " + std::to_string(b->maxN) +
                                               " particles at " + std::to_string(threads) + " threads per block");
+    // the attribute is the function's, not this batch's: the most a block can
+    // have, so that no other batch's smaller blocks lower it below this one's
+    const int most = optin > 0 ? optin - (int)stat : (int)smem;
     int resident = 0;
     cudaError_t e = cudaSuccess;
-    with_kernel(b->D, b->mixed, [&](auto k) {
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    with_kernel(b->D, b->mixed, false, [&](auto k) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k, threads, smem);
     });
     if (e != cudaSuccess) {
@@ -1198,13 +1298,42 @@ static int configure_launch(pimdb_batch* b, int threads, int ctas_per_sm) {
     b->threads = threads;
     b->ctas_per_sm = std::min(ctas_per_sm, resident);
     b->smem = smem;
-    b->grid = std::max(1, std::min(b->nrep, b->sms * b->ctas_per_sm));
+    // CTAs per replica: as many (a power of two up to 8) as leave every
+    // replica a cluster of its own among the resident CTAs, if that many
+    // clusters are resident at once
+    b->cluster = 1;
+    for (int c = kBatchMaxCluster; c > 1; c /= 2) {
+        if ((long long)b->nrep * c > (long long)b->sms * b->ctas_per_sm) continue;
+        int clusters = 0;
+        with_kernel(b->D, b->mixed, true, [&](auto k) {
+            cudaLaunchConfig_t cfg;
+            cudaLaunchAttribute at;
+            batch_config(cfg, at, b->nrep * c, threads, smem, c, b->stream);
+            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess ||
+                cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess)
+                clusters = 0;
+        });
+        cudaGetLastError();
+        if (clusters >= b->nrep) {
+            b->cluster = c;
+            break;
+        }
+    }
+    b->grid = std::max(1, std::min(b->nrep, b->sms * b->ctas_per_sm)) * b->cluster;
     return PIMDB_OK;
 }
 
 static void launch_batch(pimdb_batch* b, int mode) {
-    with_kernel(b->D, b->mixed, [&](auto k) {
-        k<<<b->grid, b->threads, b->smem, b->stream>>>(b->d_reps, b->d_order, b->nrep, b->d_ctl, b->d_step, mode);
+    with_kernel(b->D, b->mixed, b->cluster > 1, [&](auto k) {
+        if (b->cluster == 1) {
+            k<<<b->grid, b->threads, b->smem, b->stream>>>(b->d_reps, b->d_order, b->nrep, b->d_ctl, b->d_step, mode);
+            return;
+        }
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        batch_config(cfg, at, b->grid, b->threads, b->smem, b->cluster, b->stream);
+        cudaLaunchKernelEx(&cfg, k, (const BatchRep*)b->d_reps, (const int*)b->d_order, b->nrep, b->d_ctl, b->d_step,
+                           mode);
     });
     ++b->launches;
 }

@@ -424,9 +424,10 @@ __device__ inline int weights_df_block_f64arg(const Sys& s, const dfl::ExpTable&
     }
     return band;
 }
-__device__ inline int weights_df_block(const Sys& s, const dfl::ExpTable& etbl, float* vsm) {
+// Rows warp, warp + nw, ...
+__device__ inline int weights_df_block(const Sys& s, const dfl::ExpTable& etbl, float* vsm, int warp, int nw) {
     using dfl::df;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31;
     const int N = s.N;
     float* vh = vsm;               // Vh hi, lo
     float* vbh = vsm + 2 * (N + 1);  // Vbh hi, lo
