@@ -162,6 +162,53 @@ __device__ __forceinline__ void block_sum_axes(double* v, double* sh, double (*c
     __syncthreads();
 }
 
+// The same sums of the momenta as they stand, in the order one block of
+// kSumThreads threads takes them in momenta_pass and block_sum_axes, whatever
+// the team: mixed precision rounds forces to FP32, so that another order of
+// these sums (2^-53) would show as 2^-24 of a force here and there.  By the
+// first CTA; a second reading of p, about 6 us for 128 particles and 64 beads.
+constexpr int kSumThreads = 256;
+template <int D, bool kCl>
+__device__ __noinline__ void resum_axes(const Sys& s, double* v, double* sh, double (*com)[4], int& turn) {
+    const int N = s.N, H = (N + 1) / 2, total = s.P * H, lane = threadIdx.x & 31;
+    Team<kCl>::sync();  // every momentum is written
+    if (Team<kCl>::rank() == 0) {
+        for (int t = threadIdx.x; t < kSumThreads; t += blockDim.x) {
+#pragma unroll 1
+            for (int a = 0; a < D; ++a) {
+                double sa = 0.0;
+#pragma unroll 4
+                for (int q = t; q < total; q += kSumThreads) {
+                    const int b = q / H, i2 = q - b * H;
+                    const double2 p = *reinterpret_cast<const double2*>(s.p + idx<D>(s, b, a, 2 * i2));
+                    sa += p.x;
+                    if (2 * i2 + 1 < N) sa += p.y;
+                }
+                sa = warp_sum(sa);
+                if (lane == 0) sh[a * 32 + (t >> 5)] = sa;
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+        double t = 0.0;
+        for (int k = 0; k < kSumThreads / 32; ++k) t += sh[a * 32 + k];
+        v[a] = t;
+    }
+    if constexpr (kCl) {
+        double* slot = com[turn & 1];
+        ++turn;
+        if (threadIdx.x == 0)
+#pragma unroll
+            for (int a = 0; a < D; ++a) slot[a] = v[a];
+        Team<true>::sync();
+#pragma unroll
+        for (int a = 0; a < D; ++a) v[a] = Team<true>::peer(slot + a, 0);
+    }
+    __syncthreads();
+}
+
 // The normal-mode propagator's kick force of elements (b, a, i0) and
 // (b, a, i0 + 1), as the one-system path forms it (nm_kick_force): the
 // physical force, and on the bosonic end beads the exchange's spring force
@@ -1008,6 +1055,7 @@ __device__ void batch_replica(const Sys& s, int flags, const NmTabs& nm, long lo
     const bool langevin = flags & BF_LANGEVIN, fixcom = flags & BF_FIXCOM;
     const bool nmprop = flags & BF_NM, nmthermo = langevin && (flags & BF_NMTHERMO);
     const bool cart_langevin = langevin && !nmthermo;
+    const bool resum = sizeof(R) == 4 && (kCl || blockDim.x != kSumThreads);
     double* wsm = reinterpret_cast<double*>(work);  // normal-mode lines (free outside the force phase)
     const double inv_np = 1.0 / ((double)s.N * s.P);
     double cm[D], sum[D];
@@ -1019,7 +1067,8 @@ __device__ void batch_replica(const Sys& s, int flags, const NmTabs& nm, long lo
             if (nmthermo) nm_thermo_block<D, R, kCl>(s, nm, step, 0, cm, false, sum, wsm);
             else momenta_pass<D, R, kCl>(s, step, 0, cm, false, false, cart_langevin, false, sum);
             if (fixcom) {
-                block_sum_axes<D, kCl>(sum, red, com, turn);
+                if (resum && !nmthermo) resum_axes<D, kCl>(s, sum, red, com, turn);
+                else block_sum_axes<D, kCl>(sum, red, com, turn);
 #pragma unroll
                 for (int a = 0; a < D; ++a) cm[a] = sum[a] * inv_np;
             } else {
@@ -1055,7 +1104,8 @@ __device__ void batch_replica(const Sys& s, int flags, const NmTabs& nm, long lo
             momenta_pass<D, R, kCl>(s, step, 1, cm, false, true, cart_langevin, false, sum, false);
         }
         if (fixcom) {
-            block_sum_axes<D, kCl>(sum, red, com, turn);
+            if (resum && !nmthermo) resum_axes<D, kCl>(s, sum, red, com, turn);
+            else block_sum_axes<D, kCl>(sum, red, com, turn);
 #pragma unroll
             for (int a = 0; a < D; ++a) cm[a] = sum[a] * inv_np;
             momenta_pass<D, R, kCl>(s, step, 1, cm, true, false, false, false, sum);
@@ -1192,6 +1242,7 @@ struct pimdb_batch {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     int cluster = 1;  // CTAs per replica
+    bool keep_shape = false;  // mixed precision with a normal-mode thermostat
     int threads = 256, ctas_per_sm = 2, grid = 1, maxN = 1, sms = 1, maxPnm = 0;
     size_t smem = 0;
     bool use_graph = true;
@@ -1300,9 +1351,10 @@ static int configure_launch(pimdb_batch* b, int threads, int ctas_per_sm) {
     b->smem = smem;
     // CTAs per replica: as many (a power of two up to 8) as leave every
     // replica a cluster of its own among the resident CTAs, if that many
-    // clusters are resident at once
+    // clusters are resident at once.  (Not for mixed precision with the
+    // normal-mode thermostat, whose sums follow the warps: see resum_axes.)
     b->cluster = 1;
-    for (int c = kBatchMaxCluster; c > 1; c /= 2) {
+    for (int c = b->keep_shape ? 1 : kBatchMaxCluster; c > 1; c /= 2) {
         if ((long long)b->nrep * c > (long long)b->sms * b->ctas_per_sm) continue;
         int clusters = 0;
         with_kernel(b->D, b->mixed, true, [&](auto k) {
@@ -1423,6 +1475,7 @@ extern "C" int pimdb_batch_create(const pimdb_config* cfgs, int nreplicas, void*
                            (cfgs[r].fixcom ? BF_FIXCOM : 0) |
                            (cfgs[r].propagator == PIMDB_PROP_NORMAL_MODES ? BF_NM : 0) |
                            (cfgs[r].nmthermostat ? BF_NMTHERMO : 0);
+        if (b->mixed && cfgs[r].nmthermostat) b->keep_shape = true;
         b->hoff[r] = hoff;
         hoff += (size_t)s.P * s.N * D;
     }
@@ -1520,9 +1573,28 @@ extern "C" int pimdb_batch_create(const pimdb_config* cfgs, int nreplicas, void*
         free_batch(b);
         return bfail(nullptr, PIMDB_ERR_CUDA, cudaGetErrorString(e));
     }
-    // 256 threads unless the largest replica's staging needs smaller blocks
+    // Block shape (us per step, mixed / FP64, 61-512 replicas measured):
+    //  - fewer replicas than SMs: four blocks of 128 threads per SM, which
+    //    leaves the most CTAs per replica's cluster (61 replicas of up to 100
+    //    particles 174 / 216 against 194 / 268 for two of 256; 130: 362 / 491
+    //    against 390 / 570);
+    //  - else with large replicas one block of 512 (512 of up to 128: 795 /
+    //    1240 against 952 / 1374; 320 of up to 100: 432 / 689 against 716 / 1121);
+    //  - else two of 256 (512 of up to 20: 216 / 551 against 312 / 564 for one
+    //    of 512; 450 of up to 60: 363 / 661 against 387 / 688).
+    // Smaller blocks where the largest replica's staging needs them.
+    int threads = 256, ctas = 2;
+    if (b->keep_shape) {
+        threads = kSumThreads;
+    } else if (nreplicas < b->sms) {
+        threads = 128;
+        ctas = 4;
+    } else if (b->maxN > 64) {
+        threads = 512;
+        ctas = 1;
+    }
     int st = PIMDB_ERR_CONFIG;
-    for (int t = 256; t >= 32 && st == PIMDB_ERR_CONFIG; t /= 2) st = configure_launch(b, t, 2);
+    for (int t = threads; t >= 32 && st == PIMDB_ERR_CONFIG; t /= 2) st = configure_launch(b, t, ctas);
     if (st != PIMDB_OK) {
         const std::string msg = b->err;
         free_batch(b);
