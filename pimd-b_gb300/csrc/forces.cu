@@ -1562,8 +1562,17 @@ size_t pair_partial_doubles(const Sys& s, int D) { return pair_slot_doubles(s, D
 // Kernels of launch_pair_tiles_and_finish: without pairs, or with the
 // harmonic interaction of every pair in FP64 (O(N), in the finishing kernel;
 // mixed precision keeps its FP32 pair arithmetic), only the finishing one.
+// The FP64 dipole of every pair takes near/far tiles from four tiles an SM
+// (one per FP64 pipe) on: with fewer each warp has its pipe to itself, and the
+// second kernel and the near list cost more than the FP64 operations they
+// save (us a step, all FP64 / near-far: 64 particles and 16 beads 69 / 85,
+// 256 and 16 121 / 133, 192 and 32 89 / 90; 384 and 16 201 / 166, 256 and 32
+// 114 / 108, 700 and 4 311 / 297).
+constexpr long long kNearFarMinTiles = 4 * 152;
 static bool near_far_tiles(const Sys& s, int mixed) {
-    return !mixed && s.int_kind == POT_DIPOLE && s.cutoff < 0.0 && !s.pbc;
+    const long long T = (s.N + kTile - 1) / kTile;
+    return !mixed && s.int_kind == POT_DIPOLE && s.cutoff < 0.0 && !s.pbc &&
+           T * (T + 1) / 2 * s.P >= kNearFarMinTiles;
 }
 int pair_tile_kernels(const Sys& s, int mixed) {
     if (s.int_kind == POT_FREE || s.cutoff == 0.0) return 1;
