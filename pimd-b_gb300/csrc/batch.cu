@@ -488,18 +488,26 @@ __device__ void bead_forces_warp(const Sys& s, int b, int lane, unsigned char* s
     const bool dfp = sizeof(R) == 8 && (s.int_kind == POT_HARMONIC || s.int_kind == POT_DIPOLE);
     // FP64 with the harmonic interaction of every pair: from the bead's sum
     // (harmonic_all_force; an ensemble of 61 replicas of up to 100 particles:
-    // 862 us a step with the double-float pair loop, 495 us with the sum)
+    // 862 us a step with the double-float pair loop, 495 us with the sum).
+    // A plain FP64 sum: its rounding, 2^-53 of the sum of |y| an addition, is
+    // below that of the double-float pairs (2^-48 a pair), and the 8 FP64
+    // instructions of a two-sum would each take the FP64 pipe 16 cycles
+    // whatever the number of particles.
     const bool hall = sizeof(R) == 8 && pairs && harmonic_all_pairs(s);
-    double ref[D], shi[D], slo[D];
+    double ref[D], sum[D];
     if (hall) {
 #pragma unroll
         for (int a = 0; a < D; ++a) {
             const double* row = s.x + idx<D>(s, b, a, 0);
             ref[a] = row[0];
-            shi[a] = slo[a] = 0.0;
-            for (int j = lane; j < N; j += 32) add_to_pair(row[j] - ref[a], shi[a], slo[a]);
-            warp_sum_pair(shi[a], slo[a]);
+            sum[a] = 0.0;
+            for (int j = lane; j < N; j += 32) sum[a] += row[j] - ref[a];
         }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            if (o < N)  // lanes from N hold nothing, and need nothing
+#pragma unroll
+                for (int a = 0; a < D; ++a) sum[a] += __shfl_xor_sync(0xffffffffu, sum[a], o);
     } else if (pairs) {
         for (int j0 = lane; j0 < N; j0 += 32 * kStageUnroll) {
             double xs[kStageUnroll][D];
@@ -559,7 +567,7 @@ __device__ void bead_forces_warp(const Sys& s, int b, int lane, unsigned char* s
         ext_force<D>(s, xi, acc);
         if (hall) {
 #pragma unroll
-            for (int a = 0; a < D; ++a) acc[a] += harmonic_all_force(s, xi[a] - ref[a], shi[a], slo[a]);
+            for (int a = 0; a < D; ++a) acc[a] += harmonic_all_force(s, xi[a] - ref[a], sum[a], 0.0);
         } else if (pairs && dfp) {
             double g[D];
             bead_pairs_df<D>(s, b, i, xi, stage, g);
