@@ -5,7 +5,8 @@
 // The reference runs one system per MPI job (src/pimdb.cpp:31-68,
 // src/simulation.cpp:236-260); an ensemble of small systems is many jobs.
 // Here a persistent grid takes whole replicas from a work counter, largest
-// first, and one CTA runs the complete step of one replica:
+// first, and one CTA runs the complete step of one replica (with few replicas
+// a cluster of up to 8 CTAs shares it: Team):
 //   head    O-step (substep 0), COM removal, B half-kick, A drift
 //   forces  external + pair forces per bead (one warp per bead, positions
 //           staged in shared memory), interior springs, and on bosonic
@@ -16,14 +17,15 @@
 // (src/propagators/velocity_verlet.cpp:7-38) or the normal-mode one
 // (src/propagators/normal_modes_propagator.cpp:19-71) and the Langevin
 // thermostat (src/thermostats/langevin.cpp:10-27) in either frame.  Nothing
-// waits on another CTA: the only cross-CTA state is the work counter, reset
+// waits on a CTA outside its cluster: the only other shared state is the work counter, reset
 // by the CTA that finishes last, which also advances the device-side step
 // counter, so a sequence of step launches can be captured once in a CUDA
 // graph and replayed.
 //
 // Precision: `R` is the pair-force arithmetic.  R = double is the FP64 path
-// (same noise, formulas and exchange as the one-system path; harmonic and
-// dipole pairs in double-float, bead_pairs_df).  R = float computes pair
+// (same noise, formulas and exchange as the one-system path; the harmonic
+// interaction of every pair from the bead's sum, other harmonic and dipole
+// pairs in double-float, bead_pairs_df).  R = float computes pair
 // separations from hi/lo float pairs and pair gradients in FP32, sums each
 // 32-particle tile in FP32 and accumulates tiles in FP64, forms the
 // exchange weights in double-float and the exterior spring forces in FP32
@@ -166,7 +168,7 @@ __device__ __forceinline__ void block_sum_axes(double* v, double* sh, double (*c
 // kSumThreads threads takes them in momenta_pass and block_sum_axes, whatever
 // the team: mixed precision rounds forces to FP32, so that another order of
 // these sums (2^-53) would show as 2^-24 of a force here and there.  By the
-// first CTA; a second reading of p, about 6 us for 128 particles and 64 beads.
+// first CTA; a second reading of p.
 constexpr int kSumThreads = 256;
 template <int D, bool kCl>
 __device__ __noinline__ void resum_axes(const Sys& s, double* v, double* sh, double (*com)[4], int& turn) {
@@ -1584,12 +1586,17 @@ extern "C" int pimdb_batch_create(const pimdb_config* cfgs, int nreplicas, void*
     // Block shape (us per step, mixed / FP64, 61-512 replicas measured):
     //  - fewer replicas than SMs: four blocks of 128 threads per SM, which
     //    leaves the most CTAs per replica's cluster (61 replicas of up to 100
-    //    particles 174 / 216 against 194 / 268 for two of 256; 130: 362 / 491
-    //    against 390 / 570);
-    //  - else with large replicas one block of 512 (512 of up to 128: 795 /
-    //    1240 against 952 / 1374; 320 of up to 100: 432 / 689 against 716 / 1121);
-    //  - else two of 256 (512 of up to 20: 216 / 551 against 312 / 564 for one
-    //    of 512; 450 of up to 60: 363 / 661 against 387 / 688).
+    //    particles 193 / 195 against 213 / 229 for two of 256; 130: 379 / 372
+    //    against 414 / 450);
+    //  - else with large replicas one block of 512 (512 of up to 128: 786 /
+    //    995 against 936 / 1116; 320 of up to 100: 436 / 511 against 722 / 873),
+    //    and with at most two per SM from 25 particles on, where an SM's two
+    //    replicas one after the other with twice the warps each end sooner
+    //    (200 of up to 32: 158 / 184 against 190 / 241; 300 of up to 60: 282 /
+    //    346 against 360 / 477);
+    //  - else two of 256 (512 of up to 20: 216 / 249 against 289 / 341 for one
+    //    of 512; 200 of up to 20: 148 / 199 against 153 / 174; 450 of up to
+    //    60: 363 / 479 against 377 / 448).
     // Smaller blocks where the largest replica's staging needs them.
     int threads = 256, ctas = 2;
     if (b->keep_shape) {
@@ -1597,7 +1604,7 @@ extern "C" int pimdb_batch_create(const pimdb_config* cfgs, int nreplicas, void*
     } else if (nreplicas < b->sms) {
         threads = 128;
         ctas = 4;
-    } else if (b->maxN > 64) {
+    } else if (b->maxN > 64 || (b->maxN > 24 && nreplicas <= 2 * b->sms)) {
         threads = 512;
         ctas = 1;
     }
