@@ -130,12 +130,11 @@ def batched_workload(precision, n=512, seed=12345):
         ps.append(rng.normal(0.0, math.sqrt(mass / thermo_beta), (P, N, 3)))
     return cfgs, xs, ps
 
-# FP32 operations per ordered pair evaluation of the FP64 batch's
-# double-float all-pairs harmonic loop (bead_pairs_df, counted from the
-# source; FMA = 1): the separation (3 AccurateDWPlusDW, 60) and the gradient
-# sum (3 DWTimesDW + 3 AccurateDWPlusDW, 81).  The batch evaluates every
-# ordered pair (each unique pair twice).
-DF_OPS_PER_BATCH_PAIR = 141
+# FP64 FLOPs per bead, particle and axis of the FP64 batch's harmonic
+# interaction of every pair (from the bead's sum, counted from the source;
+# FMA = 2): y = x - x_0 and the sum (2), then y, S - N y, the scale and the
+# addition to the force (6).
+BATCH_HARMONIC_FLOP = 8
 
 # The exchange's FP64 accounting per evaluation: about 19 N^2 FLOPs and
 # 1.5 N^2 exponentials (cycle energies, both recursions, the exterior
@@ -171,14 +170,14 @@ def batched_roofline(cfgs, t_step, precision, peaks):
     bytes per bead-particle (x, p, f read and written) and F_exch = 19 N^2
     FP64 FLOPs per replica (its 1.5 N^2 + 0.5 N^2 exponentials are counted
     apart).  Pairs: mixed precision, 17 FLOPs per unique harmonic pair and
-    bead (FMA = 2) against the FP32 FMA peak; FP64, the double-float loop's
-    141 FP32 operations per ordered pair against the FP32 issue rate (half
-    the FMA peak in FLOP/s), with the FP64-equivalent 17 FLOPs per unique
-    pair against the FP64 peak beside it.  frac = t_ideal / t_measured."""
+    bead (FMA = 2) against the FP32 FMA peak; FP64, the 8 FLOPs per bead,
+    particle and axis of the bead's sum against the FP64 peak, with the 17
+    FLOPs per unique pair against the FP64 peak beside it.
+    frac = t_ideal / t_measured."""
     units = sum(c.natoms * c.nbeads for c in cfgs)
     B = 6 * 3 * 8 * units
     F_pair = sum(17 * c.nbeads * c.natoms * (c.natoms - 1) // 2 for c in cfgs)
-    ordered = sum(c.nbeads * c.natoms * (c.natoms - 1) for c in cfgs)
+    F_sum = BATCH_HARMONIC_FLOP * 3 * units
     F_exch = sum(19 * c.natoms ** 2 for c in cfgs)
     exps = sum(2 * c.natoms ** 2 for c in cfgs)
     bw = peaks["hbm_gbs"] * 1e9
@@ -187,7 +186,7 @@ def batched_roofline(cfgs, t_step, precision, peaks):
     if precision == "mixed":
         t_pair, pair_bound = F_pair / p32, "fp32 pipe (pairs)"
     else:
-        t_pair, pair_bound = ordered * DF_OPS_PER_BATCH_PAIR / (0.5 * p32), "fp32 pipe (double-float pairs)"
+        t_pair, pair_bound = F_sum / p64, "fp64 pipe (pairs from the bead's sum)"
     t_ideal = B / bw + t_pair + F_exch / p64
     out = {"bound": "fp64 pipe (exchange) + " + pair_bound + " + hbm",
            "t_ideal_ms": 1e3 * t_ideal, "t_measured_ms": 1e3 * t_step, "frac": t_ideal / t_step,
@@ -198,11 +197,11 @@ def batched_roofline(cfgs, t_step, precision, peaks):
            "peak_source": "HBM: MEASURED_PEAKS.json; FP64 and FP32: FMA probes measured in this run "
                           "(MEASURED_PEAKS.json has neither)"}
     if precision != "mixed":
-        out["pair_fp32_ops_per_step"] = ordered * DF_OPS_PER_BATCH_PAIR
+        out["pair_fp64_flops_per_step"] = F_sum
         t_eq = B / bw + F_pair / p64 + F_exch / p64
         out["fp64_equivalent"] = {"t_ideal_ms": 1e3 * t_eq, "frac": t_eq / t_step,
-                                  "accounting": "the same FLOPs with the pairs on the FP64 pipe; above 1: the "
-                                                "pair arithmetic no longer runs there"}
+                                  "accounting": "every pair's FLOPs on the FP64 pipe; above 1: the bead's sum "
+                                                "replaces them"}
     return out
 
 

@@ -391,9 +391,14 @@ int pimdb_exchange_noalloc(const double* ring, int nbeads, int natoms, int ndim,
  * 19-71; nbeads <= 256), and the Langevin thermostat in the cartesian or the
  * normal-mode frame, or none (Nose-Hoover chains: one system at a time).
  * Every replica must share ndim and precision; natoms <= 2048; at most 65535
- * replicas.  Blocks are 256 threads unless every warp's staged copy of the
- * largest replica needs smaller ones (above about 900 particles); a block
- * shape that cannot hold it returns PIMDB_ERR_CONFIG.  With PIMDB_MIXED the pair forces are FP32 with FP64
+ * replicas.  The default block shape follows the replica count and the
+ * largest replica: with fewer replicas than SMs four blocks of 128 threads per
+ * SM, and a cluster of up to 8 blocks per replica where they fit; else one
+ * block of 512 (more than 64 particles, or more than 24 and at most two
+ * replicas per SM) or two of 256; smaller ones where every warp's staged copy
+ * of the largest replica needs it (above about 900 particles).  A block shape
+ * that cannot hold it returns PIMDB_ERR_CONFIG.  With PIMDB_MIXED the pair
+ * forces are FP32 with FP64
  * accumulation, the exchange weights double-float and its exterior spring
  * forces FP32 with compensated sums; potentials, triangular solve, cycle
  * energies and integrator stay FP64.  The Langevin normals are the

@@ -8,7 +8,8 @@
 //   evaluateConnectionProbabilities :142-157,
 //   springForceLastBead / springForceFirstBead :159-215
 //                                           -> k_exch_forces (probabilities formed on the fly)
-//   primEstimator :250-279, getDistinctProbability :222-229,
+//   primEstimator :250-279 (as a sum over the connection probabilities),
+//   getDistinctProbability :222-229,
 //   getLongestProbability :238-240          -> k_exch_estimators
 //
 // Cycle energies are stored packed by row: the reference's E(m, k) (cycle of
@@ -20,9 +21,9 @@
 // is sequential in m and costs one FP64 exponential per term, which on one
 // streaming multiprocessor is far too slow (GB300 runs FP64 at 1/64 of FP32).
 // It is evaluated in three passes with the same result in FP64:
-//   1. k_exch_estimate: the recursion in FP32 (hardware exp2), one block,
-//      one barrier per level ("wavefront": when V[j] is final every later
-//      level adds its term u = j to a running log-sum-exp).  Gives Vh.
+//   1. k_exch_estimate / k_exch_estimate_grid (from 512 particles, across
+//      SMs): the recursion in FP32 (hardware exp2) in blocks of 32 levels.
+//      Gives Vh.
 //   2. k_exch_weights: every FP64 exponential at once, spread over the GPU:
 //      Wf[m-1][u] = exp(-beta (E[m-1][u] + Vh[u] - Vh[m])) / m.
 //   3. k_exch_solve: y_0 = 1, y_m = sum_u Wf[m-1][u] y_u (an FP64 triangular
@@ -894,7 +895,7 @@ __device__ __noinline__ void band_standalone_tail(const Sys& s, int dir, double*
 // (one warp each: inv = (I - L)^-1 and T = inv U with U the rows' weights on
 // the previous block's last cw >= band nodes), after which a right-hand side
 // is solved by a product with inv per block (side by side) and one cw-term
-// sum per block in sequence, e_b = inv rho_b + T e_{b-1}: about 100 cycles a
+// sum per block in sequence, e_b = inv rho_b + T e_{b-1}: 330 cycles a
 // block of 32 nodes.  y starts at 0 with rho the unit vector; every further
 // round takes the residual rho = W y - y in FP64 (all nodes side by side) and
 // adds the correction to y in FP64, which gains about six digits a round,

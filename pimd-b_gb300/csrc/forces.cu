@@ -1166,7 +1166,7 @@ __global__ void k_bead_finish(Sys s, const double* __restrict__ part, int T, int
 
 // The whole force evaluation with the harmonic interaction of every pair
 // (FP64; harmonic_all_pairs): one block per (bead, axis) row, its sum first.
-// N = 61, P = 20: 5 us in place of the pair tiles' 22 and k_bead_finish's 5.
+// N = 61, P = 20: 7.5 us in place of the pair tiles' 22 and k_bead_finish's 5.
 constexpr int kRowThreads = 128;
 template <int D>
 __global__ void __launch_bounds__(kRowThreads) k_bead_finish_harmonic(Sys s, int write_phys, int add_fx) {
@@ -1559,9 +1559,6 @@ static size_t pair_slot_doubles(const Sys& s, int D) {
 }
 size_t pair_partial_doubles(const Sys& s, int D) { return pair_slot_doubles(s, D) + (size_t)s.P * s.ld / 2 + 1; }
 
-// Kernels of launch_pair_tiles_and_finish: without pairs, or with the
-// harmonic interaction of every pair in FP64 (O(N), in the finishing kernel;
-// mixed precision keeps its FP32 pair arithmetic), only the finishing one.
 // The FP64 dipole of every pair takes near/far tiles from four tiles an SM
 // (one per FP64 pipe) on: with fewer each warp has its pipe to itself, and the
 // second kernel and the near list cost more than the FP64 operations they
@@ -1574,6 +1571,9 @@ static bool near_far_tiles(const Sys& s, int mixed) {
     return !mixed && s.int_kind == POT_DIPOLE && s.cutoff < 0.0 && !s.pbc &&
            T * (T + 1) / 2 * s.P >= kNearFarMinTiles;
 }
+// Kernels of launch_pair_tiles_and_finish: without pairs, or with the
+// harmonic interaction of every pair in FP64 (O(N), in the finishing kernel;
+// mixed precision keeps its FP32 pair arithmetic), only the finishing one.
 int pair_tile_kernels(const Sys& s, int mixed) {
     if (s.int_kind == POT_FREE || s.cutoff == 0.0) return 1;
     if (near_far_tiles(s, mixed)) return 3;
