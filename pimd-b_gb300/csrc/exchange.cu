@@ -784,7 +784,9 @@ __device__ __forceinline__ int finish_direction(const Sys& s, int dir, const dou
     double* V = dir == 0 ? s.V : s.Vb;
     double* yo = dir == 0 ? s.yf : s.yb;
     int flags = 0;  // 1 unusable, 2 thirty kT off, 4 not finite
-    for (int m = dir == 0 ? tid : tid + 1; m < N + (dir == 0); m += bd) {
+    // (m = 0 of direction 0 is y = 1, V = Vh: left to the thread below, so that
+    // N = bd nodes stay one pass)
+    for (int m = tid + 1; m < N + (dir == 0); m += bd) {
         const double y = ys[dir == 0 ? m : N - m];
         const double ly = log_df(y, et);
         const double v = Vh[m] - ly * s.inv_beta_ex;
@@ -794,9 +796,9 @@ __device__ __forceinline__ int finish_direction(const Sys& s, int dir, const dou
         yo[m] = y;
         V[m] = v;
     }
-    if (dir == 1 && tid == 0) {
-        V[N] = 0.0;
-        yo[N] = 1.0;
+    if (tid == bd - 1) {
+        V[dir == 0 ? 0 : N] = dir == 0 ? Vh[0] : 0.0;
+        yo[dir == 0 ? 0 : N] = 1.0;
     }
     if (flags) atomicOr(word, flags);
     __syncthreads();
@@ -818,26 +820,35 @@ __device__ __forceinline__ void finish_both(const Sys& s, int extrapolate, const
     const double VN = __ldcg(s.V + N);
     const int off = __ldcg(s.xflags + 4) | __ldcg(s.xflags + 5);
     const int order = s.Vp ? __ldcg(s.xflags + kExchOrder) : 1;
-    for (int m = tid; m <= N; m += blockDim.x) {
-        const double v = __ldcg(s.V + m), vb = m >= 1 ? __ldcg(s.Vb + m) : 0.0, vh = s.Vh[m];
-        double p = v, pb = vb;
-        bool ext = false;
-        if (s.Vp && extrapolate) {
-            p = s.Vp[m];
-            pb = s.Vp[N + 1 + m];
-            ext = isfinite(p) && isfinite(pb);
-        }
-        if (m >= 1) {
-            s.rowR[m - 1] = exp_df(-beta * (vh + vb - VN), et);
-            s.rowC[m - 1] = exp_df(-beta * (v + vb - VN), et);
-        }
+    auto estimate = [&](int m, double v, double vb, double p, double pb) {
+        const bool ext = s.Vp && extrapolate && isfinite(p) && isfinite(pb);
         s.Vh[m] = ext ? 2.0 * v - p : v;
         s.Vbh[m] = ext ? 2.0 * vb - pb : vb;
         if (s.Vp) {
             s.Vp[m] = v;
             s.Vp[N + 1 + m] = vb;
         }
+    };
+    const bool old = s.Vp && extrapolate;
+    // node 0 has no row factors: beside the others, so that N = blockDim.x
+    // nodes stay one pass (with the line in finish_direction: recursions of
+    // N = 256 43.0 -> 40.8 us)
+    double v0 = 0.0, p0 = 0.0, pb0 = 0.0;
+    if (tid == 0) {
+        v0 = __ldcg(s.V);
+        if (old) {
+            p0 = s.Vp[0];
+            pb0 = s.Vp[N + 1];
+        }
     }
+    for (int m = tid + 1; m <= N; m += blockDim.x) {
+        const double v = __ldcg(s.V + m), vb = __ldcg(s.Vb + m), vh = s.Vh[m];
+        const double p = old ? s.Vp[m] : v, pb = old ? s.Vp[N + 1 + m] : vb;
+        s.rowR[m - 1] = exp_df(-beta * (vh + vb - VN), et);
+        s.rowC[m - 1] = exp_df(-beta * (v + vb - VN), et);
+        estimate(m, v, vb, p, pb);
+    }
+    if (tid == 0) estimate(0, v0, 0.0, p0, pb0);
     __syncthreads();
     if (tid == 0) {
         s.xflags[2] = 0;
