@@ -266,10 +266,11 @@ __global__ void __launch_bounds__(kLinkBlock) k_link_carry(int N, double* __rest
 
 // The lower triangle in tiles of 16 rows and 32 columns (row tiles 2k and
 // 2k + 1 have k + 1 column tiles each), row-major: those of the flat energies
-// and of the weights, whose second copies (Et, Wb) are packed by column.  A
-// tile's transposed entries go through shared memory, so that the second copy
-// is written in runs of 16 entries (from the rows directly every entry was a
-// 32-byte sector of its own).
+// and of the weights, whose second copies (Et, Wb) are packed by column.  The
+// transposed entries are written from the registers: staged in shared memory,
+// to be written in runs, they kept these blocks off the SMs that the pair
+// tiles fill (2 steps of a liquid of 643 particles and 54 beads 1041 us with
+// the staging, 866 without; N = 4096 the same).
 constexpr int kTileRows = 16, kTileCols = 32, kTileThreads = 128;
 constexpr int kTileWarps = kTileThreads / 32, kTilePer = kTileRows / kTileWarps;  // rows per warp
 __device__ __forceinline__ void tile_of(int t, int& v0, int& u0) {
@@ -284,17 +285,6 @@ static int tile_count(int N) {
     const int M = (N + kTileRows - 1) / kTileRows, k = M / 2;
     return k * (k + 1) + (M & 1) * (k + 1);
 }
-// One tile's second copy: entry (v, u), u >= 1, to out[tri(N - u - 1) + N - 1 - v].
-__device__ __forceinline__ void tile_transposed(const double (*tile)[kTileCols + 1], int v0, int u0, int N,
-                                                double* __restrict__ out) {
-    const int row = threadIdx.x & (kTileRows - 1), c0 = threadIdx.x / kTileRows;
-#pragma unroll
-    for (int k = 0; k < kTileCols * kTileRows / kTileThreads; ++k) {
-        const int c = c0 + k * (kTileThreads / kTileRows), u = u0 + c, v = v0 + row;
-        if (u >= 1 && u <= v && v < N) out[tri(N - u - 1) + (N - 1 - v)] = tile[row][c];
-    }
-}
-
 // E and Et from the prefix sums.  Under PBC the image of x1_u nearest to xP_v
 // is chosen on FP32 differences: xP_v minus x1_u + L, x1_u or x1_u - L, each
 // rounded once per tile; within 1e-6 L of the half-box edge, where FP32 might
@@ -305,7 +295,6 @@ template <int D>
 __global__ void __launch_bounds__(kTileThreads) k_exch_energies_flat(Sys s, const double* __restrict__ Lh,
                                                                      const double* __restrict__ Ll,
                                                                      const double* __restrict__ wrap) {
-    __shared__ double tile[kTileRows][kTileCols + 1];
     const int N = s.N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int v0, u0;
     tile_of(blockIdx.x, v0, u0);
@@ -363,11 +352,9 @@ __global__ void __launch_bounds__(kTileThreads) k_exch_energies_flat(Sys s, cons
         }
         const double e = hk * (((lvh[k] - luh) + (lvl[k] - lul)) + c);
         if (u <= v) s.E[tri(v) + u] = e;
-        tile[r][lane] = e;
+        // backward node r = N - u depends on node r' = N - 1 - v
+        if (u >= 1 && u <= v && v < N) s.Et[tri(N - u - 1) + (N - 1 - v)] = e;
     }
-    __syncthreads();
-    // backward node r = N - u depends on node r' = N - 1 - v
-    tile_transposed(tile, v0, u0, N, s.Et);
 }
 
 // Pass 1: block 0 forward, block 1 backward.  Phase 0 skips (early exit)
@@ -513,7 +500,6 @@ __global__ void __launch_bounds__(kGridSolveThreads) k_exch_estimate_grid(Sys s,
 __global__ void __launch_bounds__(kTileThreads) k_exch_weights(Sys s, int phase, int tiles) {
     if (phase == 1 && ((volatile int*)s.xflags)[6] == 0) return;
     __shared__ double tbl[32];
-    __shared__ double tile[kTileRows][kTileCols + 1];
     if (threadIdx.x < 32) tbl[threadIdx.x] = kExp2Table[threadIdx.x];
     __syncthreads();
     const int N = s.N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -552,11 +538,8 @@ __global__ void __launch_bounds__(kTileThreads) k_exch_weights(Sys s, int phase,
                 if (!f64_is_zero(wf) || !f64_is_zero(wb)) band = max(band, p + 1 - u);
             }
             if (u <= p) s.Wf[tri(p) + u] = wf;
-            tile[r][lane] = wb;
+            if (u >= 1 && u <= p) s.Wb[tri(N - u - 1) + (N - 1 - p)] = wb;
         }
-        __syncthreads();
-        tile_transposed(tile, p0, u0, N, s.Wb);
-        __syncthreads();
     }
     band = __reduce_max_sync(0xffffffffu, band);
     if (lane == 0 && band > 0) atomicMax(&s.xflags[kExchBand], band);
