@@ -1149,6 +1149,9 @@ __global__ void __launch_bounds__(kBatchMaxThreads)
     if (threadIdx.x < 32) tbl[threadIdx.x] = kExp2Table[threadIdx.x];
     fill_exp_table_df(etbl);
     const long long step = *(volatile long long*)step_ctr;
+    // The first store into a peer's shared memory (`item`) must find the peer
+    // running: only a barrier of the cluster says that every CTA has started.
+    if constexpr (kCl) T::sync();
     for (;;) {
         if (T::tid() == 0) {
             const int next = atomicAdd(&ctl[0], 1);
