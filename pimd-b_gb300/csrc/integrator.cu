@@ -84,21 +84,25 @@ __global__ void k_state_out(Sys s, double* __restrict__ ox, double* __restrict__
     }
 }
 
-// The centre-of-mass sums of one launch: `part` (this thread's sums per axis)
-// to per-block slots red_out[3 blk + a].  Up to kComDirect blocks the next
-// kernel's blocks add the slots up themselves (com_mean).  With more, that sum
-// was most of k_cart_update (3072 slots at N = 4096, P = 128: 88 us a launch,
-// 14-51 us without), so the block that finishes last adds them, in order, and
-// leaves the mean momentum in red_out[3 nblk + a] (no waiting; the counter
-// behind it, red_out[3 nblk + 3], is back at 0 for the next launch).  At small
-// sizes its fence, atomic and second pass would cost more than they save.
-// A warp whose pairs all lie on one axis adds up that axis alone.
+// The centre-of-mass sums of one launch.  A `red` buffer begins with a head of
+// kComHead doubles, the mean momentum of each axis and a counter of finished
+// blocks, at the same place for every kernel that writes the buffer, whatever
+// its grid; the slots of the blocks follow.  `part` (this thread's sums per
+// axis) goes to the slots.  Up to kComDirect blocks the next kernel's blocks
+// add the slots up themselves (com_mean).  With more, that sum was most of
+// k_cart_update (3072 slots at N = 4096, P = 128: 88 us a launch, 14-51 us
+// without), so the block that finishes last adds them, in order, and leaves
+// the mean in the head (no waiting; the counter is back at 0 for the next
+// launch).  At small sizes its fence, atomic and second pass would cost more
+// than they save.  A warp whose pairs all lie on one axis adds up that axis
+// alone.
 constexpr int kComDirect = 512;
 template <int D>
 __device__ __forceinline__ void com_write(const Sys& s, const double* part, double* red_out, int blk, int nblk) {
     __shared__ double sh[3][32];
     __shared__ int is_last;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    double* slots = red_out + kComHead;
 #pragma unroll
     for (int a = 0; a < D; ++a) {
         const bool any = __any_sync(0xffffffffu, part[a] != 0.0);
@@ -109,12 +113,12 @@ __device__ __forceinline__ void com_write(const Sys& s, const double* part, doub
     if (threadIdx.x < D) {
         double t = 0.0;
         for (int k = 0; k < nw; ++k) t += sh[threadIdx.x][k];
-        red_out[3 * blk + threadIdx.x] = t;
+        slots[3 * blk + threadIdx.x] = t;
     }
     if (nblk <= kComDirect) return;
     __threadfence();
     __syncthreads();
-    unsigned* ctr = reinterpret_cast<unsigned*>(red_out + 3 * (size_t)nblk + 3);
+    unsigned* ctr = reinterpret_cast<unsigned*>(red_out + 3);
     if (threadIdx.x == 0) is_last = atomicAdd(ctr, 1u) == (unsigned)(nblk - 1);
     __syncthreads();
     if (!is_last) return;
@@ -124,12 +128,12 @@ __device__ __forceinline__ void com_write(const Sys& s, const double* part, doub
     for (int a = 0; a < D; ++a) acc[a] = 0.0;
     for (int k = threadIdx.x; k < nblk; k += blockDim.x)
 #pragma unroll
-        for (int a = 0; a < D; ++a) acc[a] += ((volatile const double*)red_out)[3 * k + a];
+        for (int a = 0; a < D; ++a) acc[a] += ((volatile const double*)slots)[3 * k + a];
     const double inv = 1.0 / ((double)s.N * (double)s.P);
 #pragma unroll
     for (int a = 0; a < D; ++a) {
         const double t = block_sum(acc[a], sh[0]) * inv;
-        if (threadIdx.x == 0) red_out[3 * (size_t)nblk + a] = t;
+        if (threadIdx.x == 0) red_out[a] = t;
     }
     if (threadIdx.x == 0) *ctr = 0u;
 }
@@ -138,7 +142,7 @@ template <int D>
 __device__ __forceinline__ void com_mean(const Sys& s, const double* red_in, int nred, double* cm) {
     if (nred > kComDirect) {
 #pragma unroll
-        for (int a = 0; a < D; ++a) cm[a] = red_in[3 * (size_t)nred + a];
+        for (int a = 0; a < D; ++a) cm[a] = red_in[a];
         return;
     }
     __shared__ double sh[3][32];
@@ -148,7 +152,7 @@ __device__ __forceinline__ void com_mean(const Sys& s, const double* red_in, int
     for (int a = 0; a < D; ++a) acc[a] = 0.0;
     for (int k = threadIdx.x; k < nred; k += blockDim.x)
 #pragma unroll
-        for (int a = 0; a < D; ++a) acc[a] += red_in[3 * k + a];
+        for (int a = 0; a < D; ++a) acc[a] += red_in[kComHead + 3 * k + a];
     const int used = min(nw, (nred + 31) >> 5);  // the warps that hold slots
     if (w < used)
 #pragma unroll

@@ -19,7 +19,8 @@ void nm_tables(int P, double omega_p, double mass, double dt, std::vector<double
 // Flags of the momentum-update kernels.  Within one launch the operations
 // run in this order: COM correction from the pending partial sums, B
 // half-kick, Langevin O-step(s), A drift, sums for the next COM removal.  The
-// sums: `red` buffers of com_doubles(nblocks) doubles, zeroed once.
+// sums: `red` buffers of com_doubles(blocks of the largest grid) doubles,
+// zeroed once, which kernels of different grids may write in turn.
 enum StepFlags : int {
     SF_COM_APPLY = 1,
     SF_LANGEVIN = 2,
@@ -190,7 +191,8 @@ void launch_state_in(const Sys& s, int D, const double* sx, const double* sp, cu
 void launch_state_out(const Sys& s, int D, double* ox, double* op, double* of, cudaStream_t st);
 int cart_update_blocks(const Sys& s, int D);
 int nm_blocks(const Sys& s, int D);
-inline size_t com_doubles(int nblocks) { return 3 * (size_t)nblocks + 4; }
+constexpr int kComHead = 4;
+inline size_t com_doubles(int nblocks) { return kComHead + 3 * (size_t)nblocks; }
 void launch_cart_update(const Sys& s, int D, int flags, const double* red_in, int nred_in, double* red_out,
                         StepRef step, int substep, int kick_nm, cudaStream_t st);
 void launch_nm_thermo(const Sys& s, int D, const double* C, const double* T, int flags, const double* red_in,
