@@ -266,21 +266,32 @@ __global__ void __launch_bounds__(128) k_pair_tiles(Sys s, double* __restrict__ 
 // FP64 dipole pairs without a cutoff: near pairs in FP64, far ones in
 // double-float.  The gradient falls as r^-4, so beyond kFarRatio times its
 // nearest neighbour's distance a pair's force is at most kFarRatio^-4 = 2^-10
-// of the nearest one's, and its double-float evaluation (2^-44 of itself) adds
-// less than 2^-54 of what the nearest pair's own FP64 rounding leaves: the sum
-// over all far pairs keeps the FP64 result's accuracy at a seventh of the cost
-// per pair (about 130 FP32 operations against 15 FP64 ones at 1/64 the rate).
-// N = 1024, P = 32, 2D: 690 us with every pair in FP64 (k_pair_tiles, bound by
-// the FP64 pipe), 157 us and 17 us for the near radii so.
+// of the nearest one's, and its double-float evaluation may be that much worse
+// than FP64: the sum over all far pairs keeps the FP64 result's accuracy at a
+// seventh of the cost per pair (about 130 FP32 operations against 15 FP64 ones
+// at 1/64 the rate).  N = 1024, P = 32, 2D: 690 us with every pair in FP64
+// (k_pair_tiles, bound by the FP64 pipe), 157 us and 17 us for the near radii
+// so.
+// The double-float coordinates are relative to the bead's particle 0 and have
+// 48 bits: with m the larger of two particles' distances from it, a separation
+// is off by at most about 2^-45 m (two coordinates and their difference) and
+// r^-4 by four times that, relative to r.  So a pair is far only from m /
+// kFarExtent on, too, which bounds the error of its force by 2^-39 of itself,
+// 2^-49 of the nearest pair's (typically 2^-4 of that: the roundings are not
+// all at their bound).  In a cloud of a few thousand particles this excludes
+// next to nothing; where particle 0 lies far outside the cloud every pair of
+// the cloud is near.  It also covers the near radii's own FP32 coordinates
+// (off by 2^-23 m).
 // A pair is far when it is so for both its particles and its distance lies
 // where double-floats have room for r^-5; anything else, NaN included, is near.
 constexpr float kFarRatio2 = 36.0f;
+constexpr float kFarExtent = 16.0f;
 constexpr float kFarMinR2 = 1e-8f, kFarMaxR2 = 1e8f;
 constexpr int kNearFarWarps = 4;
 constexpr int kNearCap = 256;  // near gradients held per warp; a tile with more is summed in chunks
 
-// nr[b ld + i] = kFarRatio^2 min_j r_ij^2, from positions relative to the
-// bead's particle 0.
+// nr[b ld + i] = max(kFarRatio min_j r_ij, m_i / kFarExtent)^2, from positions
+// relative to the bead's particle 0 (m_i the largest of their components).
 template <int D>
 __global__ void __launch_bounds__(kPairThreads) k_near_radius(Sys s, float* __restrict__ nr) {
     __shared__ float xs[D][kPairThreads];
@@ -312,7 +323,11 @@ __global__ void __launch_bounds__(kPairThreads) k_near_radius(Sys s, float* __re
             if (j0 + jj != i) best = fminf(best, r2);
         }
     }
-    if (i < s.N) nr[(size_t)b * s.ld + i] = kFarRatio2 * best;
+    float m = fabsf(xi[0]);
+#pragma unroll
+    for (int a = 1; a < D; ++a) m = fmaxf(m, fabsf(xi[a]));
+    m *= 1.0f / kFarExtent;
+    if (i < s.N) nr[(size_t)b * s.ld + i] = fmaxf(kFarRatio2 * best, m * m);
 }
 
 // |r|^-5 from r2 = |r|^2: y0 = rsqrtf(r2) has 24 bits, so y0^2 is exact in
