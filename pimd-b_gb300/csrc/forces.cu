@@ -610,7 +610,11 @@ __device__ __noinline__ double aziz_scale_value_exact(double r2, const double* t
 // (each pair's gradient times the coordinate of its first particle, not
 // wrapped) into obs[0] and obs[1].  Without a cutoff every pair is an entry.
 // Bound: the FP64 pipe, about 50 operations for a pair inside the cutoff,
-// evaluated once.  The per-particle loop it replaces took each pair from both
+// evaluated once.  The screen's thresholds are widened by a bound on its FP32
+// separations' error, 1e-6 of the largest coordinate difference there can be,
+// so that it never drops a pair or takes one for a far one wherever the
+// particles are; the cutoff and the damping radius are FP64 decisions.
+// The per-particle loop it replaces took each pair from both
 // sides, inside the cutoff or not, with CUDA's exp and sqrt: the observables
 // of N = 256, P = 64 (Aziz, cutoff L/2) took 1.47 ms a call with it, 0.26 ms
 // with the tiles.
@@ -666,10 +670,26 @@ __device__ __forceinline__ void compact_tile(const Sys& s, double* __restrict__ 
         }
     }
     // 1. FP32 screen
-    const double cut = kObs && s.cutoff < 0.0 ? (double)INFINITY : s.cutoff;
-    const float cut2f = (float)(cut * cut) * 1.0001f;
+    const bool all = kObs && s.cutoff < 0.0;  // every pair is an entry
+    const double cut = all ? (double)INFINITY : s.cutoff;
+    float cut2f = (float)(cut * cut) * 1.0001f;
     const bool aziz = s.int_kind == POT_AZIZ;
-    const float near2f = aziz ? (float)(Aziz::D * Aziz::rm * Aziz::D * Aziz::rm) * 1.0001f : -1.0f;
+    float near2f = aziz ? (float)(Aziz::D * Aziz::rm * Aziz::D * Aziz::rm) * 1.0001f : -1.0f;
+    if (kObs) {
+        float m = 0.5f * (float)s.L;  // the largest |coordinate|
+        if (!s.pbc) {
+            m = 0.0f;
+#pragma unroll
+            for (int a = 0; a < D; ++a) m = fmaxf(m, fmaxf(fabsf(xif[a]), fabsf(xjf[a])));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        }
+        // per axis 4 roundings of 2^-24 m without images, 7 with (3 of L = 2 m), times sqrt(3)
+        const float err = 2e-6f * m;
+        const float c = (float)cut + err, n = (float)(Aziz::D * Aziz::rm) + err;
+        cut2f = c * c * 1.0001f;
+        if (aziz) near2f = n * n * 1.0001f;
+    }
     const float Lf = (float)s.L, halfLf = 0.5f * (float)s.L;
     const int nj = min(kTile, s.N - jt * kTile);  // valid j lanes
     const bool ivalid = i < s.N;
@@ -696,12 +716,15 @@ __device__ __forceinline__ void compact_tile(const Sys& s, double* __restrict__ 
             }
             r2 = fmaf(d, d, r2);
         }
-        // (kObs: without a cutoff a NaN separation is an entry too)
-        const bool in = ivalid && jl < nj && (!diag || st < 16 || lane < 16) && (kObs ? !(r2 > cut2f) : r2 <= cut2f);
+        const bool in = ivalid && jl < nj && (!diag || st < 16 || lane < 16) && r2 <= cut2f;
         mask |= (unsigned)in << jl;
         const bool exact = aziz && (edge || (kDf && r2 >= shell2f));
         nmask |= (unsigned)(in && (r2 < near2f || exact)) << jl;
         xmask |= (unsigned)(in && exact) << jl;
+    }
+    if (kObs && all && ivalid) {  // NaN separations too: the steps' bits whatever r2
+        const unsigned steps = lane < 16 ? 0x1fffeu : 0xfffeu;  // 1 .. 16, from lane 16 on 1 .. 15
+        mask = (nj < 32 ? (1u << nj) - 1u : 0xffffffffu) & (diag ? __funnelshift_l(steps, steps, lane) : 0xffffffffu);
     }
     // 2. i-major layout: offsets by a warp scan of the counts
     const int icnt = __popc(mask);
