@@ -280,13 +280,16 @@ __device__ __forceinline__ double aziz_far_scale(double r2, const double* tbl) {
     return fma(ri4 * ri4, pa, -e * rinv);
 }
 // The same with the pair energy (aziz.cpp:18-54 with F = 1): v = eps [A
-// exp(-alpha r_s) - C6 ix^6 - C8 ix^8 - C10 ix^10].
+// exp(-alpha r_s) - C6 ix^6 - C8 ix^8 - C10 ix^10].  The exponential is 0 from
+// |r| = 2^20 on (and for an infinite or NaN r2, which v then holds): there
+// exp_tang256's argument leaves the range whose table index is an int.
 __device__ __forceinline__ double aziz_far_scale_value(double r2, const double* tbl, double& v) {
     constexpr double rm2 = Aziz::rm * Aziz::rm, rm6 = rm2 * rm2 * rm2, rm8 = rm6 * rm2, rm10 = rm8 * rm2;
     constexpr double e6 = Aziz::C6 * Aziz::eps * rm6, e8 = Aziz::C8 * Aziz::eps * rm8, e10 = Aziz::C10 * Aziz::eps * rm10;
     constexpr double c6 = 6.0 * e6, c8 = 8.0 * e8, c10 = 10.0 * e10;
     const double rinv = rsqrt_any(r2);
-    const double e = exp_tang256(fma(-(Aziz::alpha / Aziz::rm), r2 * rinv, kAzizLnK), tbl);
+    const double ex = exp_tang256(fma(-(Aziz::alpha / Aziz::rm), r2 * rinv, kAzizLnK), tbl);
+    const double e = __double2hiint(r2) >= (1023 + 40) << 20 ? 0.0 : ex;
     const double ri2 = rinv * rinv;
     const double ri4 = ri2 * ri2;
     // e = A alpha eps / r_m exp(-alpha r_s)
@@ -294,11 +297,14 @@ __device__ __forceinline__ double aziz_far_scale_value(double r2, const double* 
     return fma(ri4 * ri4, fma(fma(c10, ri2, c8), ri2, c6), -e * rinv);
 }
 // The general form of pair_scale_d for the Aziz potential with the energy of
-// pair_value beside it, from one exponential each.
+// pair_value beside it, from one exponential each (0 below exp(-1000): the
+// damping of nearly coincident particles and the repulsion of distant ones are
+// beyond exp_tang256's arguments).
 __device__ __forceinline__ double aziz_scale_value(double r2, const double* tbl, double& v) {
+    auto ex = [&](double x) { return x < -1000.0 ? 0.0 : exp_tang256(x, tbl); };
     const double rinv = rsqrt(r2);
     const double rs = r2 * rinv * (1.0 / Aziz::rm);
-    const double rep = Aziz::A * exp_tang256(-Aziz::alpha * rs, tbl);
+    const double rep = Aziz::A * ex(-Aziz::alpha * rs);
     double g = -Aziz::alpha * rep, u = rep;
     if (!(rs > 1.0E-7 && rs < 0.01)) {
         const double ix = Aziz::rm * rinv;  // 1 / r_scaled
@@ -309,7 +315,7 @@ __device__ __forceinline__ double aziz_scale_value(double r2, const double* tbl,
         double F = 1.0, slope = ix * pa;
         if (rs < Aziz::D) {
             const double t = Aziz::D * ix - 1.0;
-            F = exp_tang256(-t * t, tbl);
+            F = ex(-t * t);
             slope -= 2.0 * Aziz::D * ix2 * t * pb;
         }
         g = fma(F * ix6, slope, g);
