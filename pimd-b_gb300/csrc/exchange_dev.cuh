@@ -373,27 +373,55 @@ __device__ inline void weights_direction(const Sys& s, int dir, const double* tb
 // weights_df_block_f64arg forms the argument in FP64 (only the exponential
 // in double-float): E, Vh_u and Vh_{p+1} are up to beta_ex V_B ~ 10^3-10^4 kT
 // and nearly cancel, so 48 bits of each leave 1e-11 in the weight.  Entries
-// whose FP32 argument is below -89 are zero without any FP64 operation.
+// whose FP32 argument is below -89 by more than its own roundings (below 3e-7
+// of its terms) are zero without any FP64 operation.
+// That an entry at -89 does not count takes a row whose largest is near 0: an
+// estimate that follows the energies to a few kT.  It is formed from 20 bits
+// of them, so potentials above kWideKT may be off by more (rings stretched far
+// beyond equilibrium): weights_wide then.
+constexpr double kWideKT = 4194304.0;  // 2^22: 2^-20 of it, a few times, is about 16 kT
+// The weights with CUDA's exp over its whole range (out of line: a rare path).
+static __device__ __noinline__ int weights_wide(const Sys& s) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int N = s.N;
+    const double nbeta = -s.beta_ex;
+    int band = 0;
+    for (int p = warp; p < N; p += nw) {
+        const double inv = recip_row(p), vp = s.Vh[p + 1], vbp = s.Vbh[p + 1];
+        for (int u = lane; u <= p; u += 32) {
+            const double E = __ldcg(s.E + tri(p) + u);
+            const double wf = exp(nbeta * (E + s.Vh[u] - vp)) * inv;
+            const double wb = u >= 1 ? exp(nbeta * (E + vbp - s.Vbh[u])) * inv : 0.0;
+            s.Wf[tri(p) + u] = wf;
+            if (u >= 1) s.Wb[tri(N - u - 1) + (N - 1 - p)] = wb;
+            if (wf != 0.0 || wb != 0.0) band = max(band, p + 1 - u);
+        }
+    }
+    return band;
+}
 __device__ inline int weights_df_block_f64arg(const Sys& s, const dfl::ExpTable& etbl, float* vsm) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int N = s.N;
     double* vh = reinterpret_cast<double*>(vsm);
     double* vbh = vh + N + 1;
+    const double nbeta = -s.beta_ex;
+    const float nbf = round_f32(nbeta);
+    int wide = 0;
     for (int m = threadIdx.x; m <= N; m += blockDim.x) {
         vh[m] = s.Vh[m];
         vbh[m] = s.Vbh[m];
+        if (!(fabs(nbeta * vh[m]) <= kWideKT && fabs(nbeta * vbh[m]) <= kWideKT)) wide = 1;
     }
-    __syncthreads();
-    const double nbeta = -s.beta_ex;
-    const float nbf = round_f32(nbeta);
+    if (__syncthreads_or(wide)) return weights_wide(s);
     int band = 0;
     for (int p = warp; p < N; p += nw) {
         const dfl::df inv = split_df(recip_row(p));
         const double vp = vh[p + 1], vbp = vbh[p + 1];
         const float vpf = round_f32(vp), vbpf = round_f32(vbp);
         const size_t r = tri(p);
-        auto weight = [&](double E, double a, double b, float quick) {
-            if (quick < -89.0f) return 0.0;
+        auto weight = [&](double E, double a, double b, float Ef, float af, float bf) {
+            const float quick = Ef + (af - bf) - 4e-7f * (fabsf(Ef) + fabsf(af) + fabsf(bf));
+            if (nbf * quick < -89.0f) return 0.0;
             const double x = nbeta * (E + a - b);
             return df_to_f64(dfl::mul(dfl::exp(split_df(x), etbl), inv));
         };
@@ -409,12 +437,12 @@ __device__ inline int weights_df_block_f64arg(const Sys& s, const dfl::ExpTable&
                 if (u > p) break;
                 const double vu = vh[u];
                 const float Ef = round_f32(E[k]);
-                const double wf = weight(E[k], vu, vp, nbf * (Ef + (round_f32(vu) - vpf)));
+                const double wf = weight(E[k], vu, vp, Ef, round_f32(vu), vpf);
                 s.Wf[r + u] = wf;
                 bool nz = !f64_is_zero(wf);
                 if (u >= 1) {
                     const double vbu = vbh[u];
-                    const double wb = weight(E[k], vbp, vbu, nbf * (Ef + (vbpf - round_f32(vbu))));
+                    const double wb = weight(E[k], vbp, vbu, Ef, vbpf, round_f32(vbu));
                     s.Wb[tri(N - u - 1) + (N - 1 - p)] = wb;
                     nz = nz || !f64_is_zero(wb);
                 }
