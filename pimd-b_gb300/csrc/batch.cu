@@ -569,7 +569,7 @@ __device__ void bead_forces_warp(const Sys& s, int b, int lane, unsigned char* s
         ext_force<D>(s, xi, acc);
         if (hall) {
 #pragma unroll
-            for (int a = 0; a < D; ++a) acc[a] += harmonic_all_force(s, xi[a] - ref[a], sum[a], 0.0);
+            for (int a = 0; a < D; ++a) acc[a] += s.int_a * fma(-(double)N, xi[a] - ref[a], sum[a]);
         } else if (pairs && dfp) {
             double g[D];
             bead_pairs_df<D>(s, b, i, xi, stage, g);

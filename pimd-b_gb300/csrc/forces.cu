@@ -1213,8 +1213,15 @@ __global__ void __launch_bounds__(kRowThreads) k_bead_finish_harmonic(Sys s, int
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const double* row = s.x + idx<D>(s, b, a, 0);
     const double ref = row[0];
-    double hi = 0.0, lo = 0.0;
-    for (int i = threadIdx.x; i < s.N; i += kRowThreads) add_to_pair(row[i] - ref, hi, lo);
+    double y = 0.0, yl = 0.0;  // this thread's first particle
+    if (threadIdx.x < s.N) two_diff_f64(row[threadIdx.x], ref, y, yl);
+    double hi = y, lo = yl;
+    for (int i = threadIdx.x + kRowThreads; i < s.N; i += kRowThreads) {
+        double v, vl;
+        two_diff_f64(row[i], ref, v, vl);
+        add_to_pair(v, hi, lo);
+        lo += vl;
+    }
     warp_sum_pair(hi, lo);
     if (lane == 0) {
         sh[warp] = hi;
@@ -1240,7 +1247,8 @@ __global__ void __launch_bounds__(kRowThreads) k_bead_finish_harmonic(Sys s, int
                 x = xi[c];
                 acc = fe[c];
             }
-        finish_component<D>(s, b, a, i, x, acc + harmonic_all_force(s, x - ref, hi, lo), write_phys, add_fx);
+        if (i >= kRowThreads) two_diff_f64(x, ref, y, yl);
+        finish_component<D>(s, b, a, i, x, acc + harmonic_all_force(s, y, yl, hi, lo), write_phys, add_fx);
     }
 }
 
