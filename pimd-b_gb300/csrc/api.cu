@@ -450,9 +450,10 @@ extern "C" int pimdb_create(const pimdb_config* cfg, void* cuda_stream, pimdb_ha
         if (e == cudaSuccess) e = cudaMemset(h->d_gflags, 0, exchange_grid_flags(s) * sizeof(unsigned));
     }
     // Newton's-third-law pair tiles need P * ceil(N/32) * D * ld partial sums;
-    // beyond 512 MiB the all-pairs kernel (no partials) is used instead.
-    const size_t npart = pair_partial_doubles(s, h->D);
-    if (e == cudaSuccess && npart * sizeof(double) <= (512ull << 20)) e = alloc(&h->d_part, npart);
+    // when these (not what else the buffer holds) and the task counters exceed
+    // 512 MiB the all-pairs kernel (no partials) is used instead.
+    if (e == cudaSuccess && (pair_slot_doubles(s, h->D) + 1) * sizeof(double) <= (512ull << 20))
+        e = alloc(&h->d_part, pair_partial_doubles(s, h->D));
     if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_step, sizeof(long long));
     h->cell_nc = cell_grid(s, h->D);
     if (e == cudaSuccess && h->cell_nc > 0) e = cudaMalloc(&h->d_cells, cell_buffer_bytes(s, h->D, h->cell_nc));

@@ -1600,7 +1600,7 @@ void launch_pair_cells_and_finish(const Sys& s, int D, int nc, int mixed, int wr
 // The partial sums, the near radii of the dipole tiles (floats) and one
 // trailing double that holds the compact kernel's two task counters (zero
 // between launches).
-static size_t pair_slot_doubles(const Sys& s, int D) {
+size_t pair_slot_doubles(const Sys& s, int D) {
     return (size_t)s.P * ((s.N + kTile - 1) / kTile) * D * s.ld;
 }
 size_t pair_partial_doubles(const Sys& s, int D) { return pair_slot_doubles(s, D) + (size_t)s.P * s.ld / 2 + 1; }

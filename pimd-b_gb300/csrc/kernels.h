@@ -41,6 +41,7 @@ void launch_bead_forces(const Sys& s, int D, int mixed, int write_phys, cudaStre
 // forces (fx) on beads 1 and P, after waiting for `before_finish` (may be
 // null) that marks them done.
 size_t pair_partial_doubles(const Sys& s, int D);
+size_t pair_slot_doubles(const Sys& s, int D);  // the partial sums alone
 // Kernels launch_pair_tiles_and_finish launches.
 int pair_tile_kernels(const Sys& s, int mixed);
 // pimdb_math_check's kernel (device arrays; out holds 8 n doubles).
