@@ -33,8 +33,8 @@
 // minima and q the columns' minima of the rest: every factor is then at most
 // 1, and the shift joins V_B again.  Where even the best permutation falls
 // below 1e-200 (links that compete for the same near targets, far from
-// equilibrium), r and q become the potentials of the optimal assignment (the
-// Hungarian algorithm, one thread): the best permutation then has weight 1.
+// equilibrium), r and q become the potentials of the optimal assignment: the
+// best permutation then has weight 1.
 // (The reference's unshifted effectivePotential underflows to V_B = inf.)
 //
 // One block; F and B (64 KB at N = 12) in shared memory, one barrier per
@@ -59,60 +59,55 @@ __host__ __device__ constexpr double factorial_of(int n) {
     return r;
 }
 
-// The optimal assignment's potentials (Kuhn's Hungarian method in the
-// shortest-augmenting-path form): r[i] + q[j] <= a[i][j] with equality on the
-// optimum.  One thread; every loop is bounded by N.
-__device__ __noinline__ void assignment_potentials(int N, const double* a, double* r, double* q) {
-    double u[kFactMaxN + 1], v[kFactMaxN + 1], minv[kFactMaxN + 1];
-    int owner[kFactMaxN + 1], way[kFactMaxN + 1];
-    for (int j = 0; j <= N; ++j) {
-        u[j] = v[j] = 0.0;
-        owner[j] = 0;
-    }
-    for (int i = 1; i <= N; ++i) {
-        owner[0] = i;
-        int j0 = 0;
-        unsigned used = 0;
-        for (int j = 0; j <= N; ++j) minv[j] = 1.79769313486231570815e308;
-        for (int it = 0; it <= N; ++it) {
-            used |= 1u << j0;
-            const int i0 = owner[j0];
-            double delta = 1.79769313486231570815e308;
-            int j1 = 0;
-            for (int j = 1; j <= N; ++j) {
-                if (used >> j & 1u) continue;
-                const double cur = a[(i0 - 1) * N + j - 1] - u[i0] - v[j];
-                if (cur < minv[j]) {
-                    minv[j] = cur;
-                    way[j] = j0;
-                }
-                if (minv[j] < delta) {
-                    delta = minv[j];
-                    j1 = j;
-                }
+// Potentials r, q with r[l] + q[m] <= a[l][m], and equality on the cheapest
+// permutation, by the whole block; `cost` (2^N doubles) is scratch.  The
+// cheapest way to place the first |c| links on the targets c is found over
+// subsets as F is, with minima for sums (dynamic programming over subsets:
+// Held and Karp 1962), and the permutation sigma by walking it back.  With
+// q[sigma(k)] = a[k][sigma(k)] - r[k] what remains are bounds on differences,
+// r[l] - r[k] <= a[l][sigma(k)] - a[k][sigma(k)], which shortest paths satisfy
+// (Bellman-Ford, N rounds: the cheapest permutation leaves no negative cycle).
+__device__ __noinline__ void assignment_potentials(int N, const double* a, double* cost, int* sigma, double* r,
+                                                   double* q) {
+    const int tid = threadIdx.x, size = 1 << N;
+    for (int n = 0; n <= N; ++n) {
+        for (int c = tid; c < size; c += kFactThreads) {
+            if (__popc(c) != n) continue;
+            double least = n ? (double)INFINITY : 0.0;
+            for (int w = c; w; w &= w - 1) {
+                const int m = __ffs(w) - 1;
+                least = fmin(least, cost[c ^ (1 << m)] + a[(n - 1) * N + m]);
             }
-            if (j1 == 0) break;  // non-finite costs: the caller's sum stays non-finite
-            for (int j = 0; j <= N; ++j) {
-                if (used >> j & 1u) {
-                    u[owner[j]] += delta;
-                    v[j] -= delta;
-                } else {
-                    minv[j] -= delta;
-                }
-            }
-            j0 = j1;
-            if (owner[j0] == 0) break;
+            cost[c] = least;
         }
-        for (int it = 0; it <= N && j0; ++it) {
-            const int j1 = way[j0];
-            owner[j0] = owner[j1];
-            j0 = j1;
+        __syncthreads();
+    }
+    if (tid < 32) {
+        if (tid == 0)
+            for (int l = N - 1, c = size - 1; l >= 0; --l) {
+                int take = __ffs(c) - 1;
+                for (int w = c & (c - 1); w; w &= w - 1) {
+                    const int m = __ffs(w) - 1;
+                    if (cost[c ^ (1 << m)] + a[l * N + m] < cost[c ^ (1 << take)] + a[l * N + take]) take = m;
+                }
+                sigma[l] = take;
+                c ^= 1 << take;
+            }
+        __syncwarp();
+        const int l = tid < N ? tid : 0;
+        double d = 0.0;
+        for (int round = 0; round < N; ++round) {
+            if (tid < N) r[tid] = d;
+            __syncwarp();
+            for (int k = 0; k < N; ++k) d = fmin(d, r[k] + (a[l * N + sigma[k]] - a[k * N + sigma[k]]));
+            __syncwarp();
+        }
+        if (tid < N) {
+            r[tid] = d;
+            q[sigma[tid]] = a[tid * N + sigma[tid]] - d;
         }
     }
-    for (int i = 0; i < N; ++i) {
-        r[i] = u[i + 1];
-        q[i] = v[i + 1];
-    }
+    __syncthreads();
 }
 
 // The sum over permutations, the scalars and the exterior spring forces of
@@ -125,6 +120,7 @@ __global__ void __launch_bounds__(kFactThreads) k_factorial(Sys s, int accumulat
     __shared__ double A[kFactMaxN * kFactMaxN];
     __shared__ double M[kFactMaxN * kFactMaxN];
     __shared__ double r[kFactMaxN], q[kFactMaxN];
+    __shared__ int sigma[kFactMaxN];
     const int tid = threadIdx.x, N = s.N, NN = N * N, size = 1 << N;
     const int lane = tid & 31, warp = tid >> 5, nw = kFactThreads / 32;
     double* F = sub;
@@ -195,8 +191,7 @@ __global__ void __launch_bounds__(kFactThreads) k_factorial(Sys s, int accumulat
         const double S = F[size - 1];
         if (S >= kFactSmallest || !isfinite(S) || attempt) break;  // the whole block alike
         __syncthreads();
-        if (tid == 0) assignment_potentials(N, ar, r, q);
-        __syncthreads();
+        assignment_potentials(N, ar, F, sigma, r, q);
     }
     const double S = F[size - 1], invS = 1.0 / S;
     // M[l][m]: one warp per entry over the subsets without m
