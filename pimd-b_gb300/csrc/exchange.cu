@@ -881,7 +881,7 @@ __device__ __noinline__ void band_standalone_tail(const Sys& s, int dir, double*
     }
 }
 
-// The banded solve by FP32 elimination with FP64 residuals (bands up to 32).
+// The banded solve by FP32 elimination with FP64 residuals (bands up to 24).
 // One warp issues an FP64 instruction every 64 cycles and a dependent
 // multiply-add takes 65 (measured), so the chain over the nodes in FP64 costs
 // 111 cycles a node whatever its arrangement.  Here each 32-node block's
@@ -892,21 +892,26 @@ __device__ __noinline__ void band_standalone_tail(const Sys& s, int dir, double*
 // sum per block in sequence, e_b = inv rho_b + T e_{b-1}: 330 cycles a
 // block of 32 nodes.  y starts at 0 with rho the unit vector; every further
 // round takes the residual rho = W y - y in FP64 (all nodes side by side) and
-// adds the correction to y in FP64, which gains about six digits a round,
-// until the last correction is below 1e-10: three rounds, and the result's
-// error is that of an FP64 residual, as in the substitution.  Gives up (false;
+// adds the correction to y in FP64.  What a round leaves is FP32's rounding
+// along the chain of the correction it adds (some 1e-5 of it), so after one
+// below 1e-10, in general the third or fourth, the error is that of an FP64
+// residual: V differs from extended precision as much as with the substitution
+// (N = 2016 to 4096, six temperatures: 1e-11 to 2e-10 kT).  Gives up (false;
 // block-uniform) where y leaves [1e-20, 1e20], so that corrections of 1e-16
 // still are FP32 numbers, or does not converge.
 // `Ls`: kBandThreads / 32 x 1024 floats; `fs`: 32 nb floats; `store`: nb
 // blocks of T [32][cw + 1] and inv [32][36].
 constexpr int kBandWarps = kBandThreads / 32;
-constexpr int kBandRefined = 32;    // the band it takes
-// Blocks from which it is the faster form: its code is long and runs once, so
-// few blocks pay more for fetching it than they save (steps of N = 256, 9
-// blocks, and N = 1024, 33 blocks, 2-3% slower with it; N = 4096, 129 blocks,
-// 8.21 -> 7.82 ms for 4 steps).
+// The band it takes, and the blocks from which it is the faster form: its code
+// is long and runs once, so few blocks pay more for fetching it than they save
+// (steps of N = 256, 9 blocks, and N = 1024, 33 blocks, 2-3% slower with it;
+// N = 4096, 129 blocks, 8.21 -> 7.82 ms for 4 steps).  Recursions, us,
+// substitution / refined, at bands of 28, 24, 19 and 13: N = 2016 298 / 309,
+// 296 / 285, 291 / 272, 287 / 260; N = 2450 352 / 384, 348 / 296, 347 / 293,
+// 340 / 278; N = 3100 435 / 443, 431 / 432, 426 / 412, 419 / 350.
+constexpr int kBandRefined = 24;
 constexpr int kBandRefinedMin = 64;
-constexpr int kBandStore = 32 * 33 + 32 * 36;  // floats per block at most (behind ysol)
+constexpr int kBandStore = 32 * 25 + 32 * 36;  // floats per block at most (behind ysol)
 // A double rounded to float by bit patterns, 0 below 2^-126 and infinite above
 // a float's range (the conversion instruction takes the FP64 pipe for 128
 // cycles a warp).
@@ -1044,8 +1049,7 @@ __device__ __noinline__ bool band_refined(const double* __restrict__ W, int nn, 
         if (warp == 0) {
             if (cw == 8) band_sequence<8>(nb, fs, store, lane);
             else if (cw == 16) band_sequence<16>(nb, fs, store, lane);
-            else if (cw == 24) band_sequence<24>(nb, fs, store, lane);
-            else band_sequence<32>(nb, fs, store, lane);
+            else band_sequence<24>(nb, fs, store, lane);
         }
         __syncthreads();
         int more = 0, bad = 0;

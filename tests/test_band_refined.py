@@ -1,7 +1,7 @@
 """The banded exchange solve by FP32 elimination with FP64 residuals, which
-takes bands up to 32 from 64 blocks of 32 nodes on (V has N + 1 nodes, V_back-
+takes bands up to 24 from 64 blocks of 32 nodes on (V has N + 1 nodes, V_back-
 wards N: at 2015 particles only V, at 2016 both), around those sizes and at
-ragged ones, with a band for each of its column widths 8, 16, 24 and 32 and one
+ragged ones, with a band for each of its column widths 8, 16 and 24 and two
 beyond, which the FP64 substitution takes; and after jumps of the coordinates,
 which put y out of the range of the FP32 corrections.  V and V_backwards
 against the recursion in extended precision over the entries within 90 nodes
