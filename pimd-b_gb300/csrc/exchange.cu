@@ -24,7 +24,7 @@
 //   1. k_exch_estimate / k_exch_estimate_grid (from 512 particles, across
 //      SMs): the recursion in FP32 (hardware exp2) in blocks of 32 levels.
 //      Gives Vh.
-//   2. k_exch_weights: every FP64 exponential at once, spread over the GPU:
+//   2. k_exch_weights_rows, k_exch_weights: every FP64 exponential at once, spread over the GPU:
 //      Wf[m-1][u] = exp(-beta (E[m-1][u] + Vh[u] - Vh[m])) / m.
 //   3. k_exch_solve: y_0 = 1, y_m = sum_u Wf[m-1][u] y_u (an FP64 triangular
 //      solve, multiply-adds only) and V[m] = Vh[m] - log(y_m)/beta exactly.
@@ -489,14 +489,35 @@ __global__ void __launch_bounds__(kGridSolveThreads) k_exch_estimate_grid(Sys s,
     }
 }
 
-// Pass 2: every FP64 exponential at once, by tiles (grid-stride; phase 1 runs
-// only on a retry).  Also records the band of the weights (kExchBand: the
-// largest p + 1 - u of a nonzero weight) for the banded solve; one atomic per
-// warp.  An entry whose FP32 argument, with the roundings of E and the two
-// potentials added, is below -701 is exactly zero (exp_tang's) without any
-// FP64 operation: nearly all of them in a large liquid (N = 4096: 245 -> 114 us
-// against one row per block without the test; where no entry is zero the FP64
-// pipe bounds either form, 23 -> 34 us at N = 777).
+// Pass 2: every FP64 exponential at once, one thread per packed entry
+// (grid-stride over rows; phase 1 runs only on a retry).  Also records the band
+// of the weights (kExchBand: the largest p + 1 - u of a nonzero weight) for the
+// banded solve; one atomic per warp.
+__global__ void __launch_bounds__(256) k_exch_weights_rows(Sys s, int phase) {
+    if (phase == 1 && ((volatile int*)s.xflags)[6] == 0) return;
+    __shared__ double tbl[32];
+    if (threadIdx.x < 32) tbl[threadIdx.x] = kExp2Table[threadIdx.x];
+    __syncthreads();
+    int band = 0;
+    for (int p = blockIdx.y; p < s.N; p += gridDim.y) {
+        const double inv = recip_row(p);
+        for (int u = blockIdx.x * blockDim.x + threadIdx.x; u <= p; u += gridDim.x * blockDim.x)
+            if (exch_weight(s, p, u, inv, tbl)) band = max(band, p + 1 - u);
+    }
+    band = __reduce_max_sync(0xffffffffu, band);
+    if ((threadIdx.x & 31) == 0 && band > 0) atomicMax(&s.xflags[kExchBand], band);
+}
+// The same by tiles, for large systems.  An entry whose FP32 argument, with the
+// roundings of E and the two potentials added, is below -701 is exactly zero
+// (exp_tang's) without any FP64 operation: nearly all of them in a large liquid
+// (N = 4096: 245 -> 114 us).  Each thread takes four entries in turn, so below
+// kTileWeightsMinN, where that leaves few warps, the row form's one entry a
+// thread hides its latencies better, above all beside the pair tiles (steps of
+// a liquid, 14 and 24 beads, us, rows / tiles: N = 512 145 / 159 and 157 / 181,
+// N = 692 190 / 208 and 206 / 220).  Recursions alone, us, liquid and (no
+// weight zero) trap: N = 767 106 / 108 and 225 / 229, N = 1100 175 / 178 and
+// 232 / 240, N = 1500 228 / 220 and 307 / 305, N = 4096 553 / 421 and 933 / 813.
+constexpr int kTileWeightsMinN = 1280;
 __global__ void __launch_bounds__(kTileThreads) k_exch_weights(Sys s, int phase, int tiles) {
     if (phase == 1 && ((volatile int*)s.xflags)[6] == 0) return;
     __shared__ double tbl[32];
@@ -1293,7 +1314,7 @@ static void exchange_carveouts() {
                        (const void*)k_link_prefix<2>, (const void*)k_link_prefix<3>, (const void*)k_link_carry,
                        (const void*)k_exch_energies_flat<1>, (const void*)k_exch_energies_flat<2>,
                        (const void*)k_exch_energies_flat<3>, (const void*)k_exch_estimate, (const void*)k_exch_estimate_grid,
-                       (const void*)k_exch_weights, (const void*)k_exch_solve, (const void*)k_exch_solve_grid,
+                       (const void*)k_exch_weights, (const void*)k_exch_weights_rows, (const void*)k_exch_solve, (const void*)k_exch_solve_grid,
                        (const void*)k_exch_forces<1>, (const void*)k_exch_forces<2>, (const void*)k_exch_forces<3>};
     for (const void* f : k)
         cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -1425,7 +1446,9 @@ int launch_exchange_recursions(const Sys& s, int exact, cudaStream_t st, double*
         k_exch_solve<<<2, kWaveThreads, smem, st>>>(s, 1, 0, nullptr, 0);
         return 1;
     }
-    const int tiles = tile_count(s.N);  // the retry's weights: a small grid-stride launch
+    // weights: rows or tiles by size; the retry's a small grid-stride launch
+    const int tiles = tile_count(s.N);
+    const dim3 wgrid((s.N + 255) / 256, s.N), rgrid(1, std::min(s.N, 256));
     // below the multi-SM solve's size a failed solve is retried inside
     // k_exch_solve (phase 0 only)
     const int inline_retry = s.N < kGridSolveMinN;
@@ -1440,7 +1463,10 @@ int launch_exchange_recursions(const Sys& s, int exact, cudaStream_t st, double*
             ++n;
         }
         if (!(phase == 0 && estimate_done)) {  // else the energy kernel formed them
-            k_exch_weights<<<phase ? std::min(tiles, 512) : tiles, kTileThreads, 0, st>>>(s, phase, tiles);
+            if (s.N < kTileWeightsMinN)
+                k_exch_weights_rows<<<phase ? rgrid : wgrid, 256, 0, st>>>(s, phase);
+            else
+                k_exch_weights<<<phase ? std::min(tiles, 512) : tiles, kTileThreads, 0, st>>>(s, phase, tiles);
             ++n;
         }
         // the banded kernel (one CTA per direction): below the multi-SM
