@@ -762,7 +762,6 @@ static void enqueue_forces(pimdb_handle* h) {
                                          fx_in_finish, h->stream);
         }, 3);
     } else if (tiles) {
-        const bool pairs = s.int_kind != PIMDB_POT_FREE && s.cutoff != 0.0;
         launch(
             h, PIMDB_K_BEAD_FORCES,
             [&] {

@@ -1290,11 +1290,14 @@ __global__ void __launch_bounds__(kEstimatorThreads) k_exch_estimators(Sys s, in
     }
 }
 
-// Every exchange kernel takes the largest shared-memory carveout.  An SM runs
-// all its resident blocks under one carveout, so a kernel that prefers a
-// smaller one (more L1) could start only on SMs without pair-tile blocks,
-// and the pair tiles' blocks could not start beside it: launched first in a
-// step graph, the exchange would hold back part of the pair kernel.
+// The exchange kernels that spread over the GPU take the largest shared-memory
+// carveout.  An SM runs all its resident blocks under one carveout, so a kernel
+// that prefers a smaller one (more L1) could start only on SMs without
+// pair-tile blocks, and the pair tiles' blocks could not start beside it:
+// launched first in a step graph, the exchange would hold back part of the pair
+// kernel.  k_exch_solve_band has two blocks and SMs of its own, and
+// k_exch_estimators comes last on its stream: with them listed too, steps and
+// observables of 100 to 692 particles took the same time.
 // Attributes belong to the current device: they are set once per device (a
 // bit per device id below 64, every call above), and two host threads that
 // set them at once only repeat the same cheap calls.
@@ -1358,7 +1361,7 @@ int launch_exchange_energies(const Sys& s, int D, cudaStream_t st, double* work)
         return 0;
     }
     // one block per row; scans [N] and two chunk arrays in shared memory
-    // (or the estimate's 3 (N + 1) floats)
+    // (or the 6 (N + 1) floats of both directions' estimate)
     const size_t rs = energies_rows_smem(s);
     if (energies_by_rows(s, work)) {
         if (D == 1) k_exch_energies_rows<1><<<s.N, kEnergyRowThreads, rs, st>>>(s);

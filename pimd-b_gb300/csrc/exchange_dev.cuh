@@ -643,7 +643,7 @@ __device__ inline int solve_direction(const Sys& s, int dir, int force_exact, do
 // 2 V(t) - V(t - dt), which smooth dynamics keep much closer.  The caller
 // asks for no extrapolation after an evaluation from a fresh estimate: the
 // coordinates may have jumped, and 2 V - V(before the jump) would fail again
-// (one more fresh estimate, 10 ms at N = 4096).  An estimate that was not
+// (one more fresh estimate, 0.63 ms at N = 4096).  An estimate that was not
 // extrapolated and is 30 kT off asks for no fresh one either: the next, which
 // is, will be far closer.  With `et` the row exponentials in double-float
 // (exp_df).

@@ -1606,7 +1606,7 @@ size_t pair_slot_doubles(const Sys& s, int D) {
 size_t pair_partial_doubles(const Sys& s, int D) { return pair_slot_doubles(s, D) + (size_t)s.P * s.ld / 2 + 1; }
 
 // The FP64 dipole of every pair takes near/far tiles from four tiles an SM
-// (one per FP64 pipe) on: with fewer each warp has its pipe to itself, and the
+// (one per FP64 pipe; a GB300 has 152 SMs) on: with fewer each warp has its pipe to itself, and the
 // second kernel and the near list cost more than the FP64 operations they
 // save (us a step, all FP64 / near-far: 64 particles and 16 beads 69 / 85,
 // 256 and 16 121 / 133, 192 and 32 89 / 90; 384 and 16 201 / 166, 256 and 32
