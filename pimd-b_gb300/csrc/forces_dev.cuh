@@ -31,7 +31,14 @@ static __constant__ double kExp2Table[32] = {
     0x1.ae89f995ad3adp+0, 0x1.b7f76f2fb5e47p+0, 0x1.c199bdd85529cp+0, 0x1.cb720dcef9069p+0,
     0x1.d5818dcfba487p+0, 0x1.dfc97337b9b5fp+0, 0x1.ea4afa2a490dap+0, 0x1.f50765b6e4540p+0};
 
+// x <= -1024, -infinity included and NaN not, by the upper word: exp(x) is 0
+// there, and far enough down (-4.6e7, with 256 entries -5.8e6) n no longer is
+// an int.  Cycles with a particle thrown far out cost that much.
+__device__ __forceinline__ bool below_exp_range(double x) {
+    return (unsigned)__double2hiint(x) - 0xc0900000u <= 0xfff00000u - 0xc0900000u;
+}
 __device__ __forceinline__ double exp_tang(double x, const double* tbl) {
+    if (below_exp_range(x)) return 0.0;
     const double shifter = 6755399441055744.0;  // 1.5 * 2^52
     const double t = fma(x, 46.16624130844683, shifter);  // 32 / ln2
     const int n = __double2loint(t);
