@@ -240,7 +240,10 @@ __device__ __forceinline__ double pair_scale_d(int kind, double r2, double param
     const double rs = norm * (1.0 / Aziz::rm);
     const double T1 = -Aziz::A * Aziz::alpha * ex(-Aziz::alpha * rs);
     double g;
-    if (rs > 1.0E-7 && rs < 0.01) {
+    // The reference leaves the attraction out from 1e-7 to 0.01; below, its
+    // damping factor exp(-(D / r_s - 1)^2) is 0 as well (and beyond
+    // exp_tang256's arguments), down to where 1 / r_s^10 overflows.
+    if (rs > 1.0E-30 && rs < 0.01) {
         g = T1 * (Aziz::eps / Aziz::rm);
     } else {
         const double ix = Aziz::rm * rinv;  // 1 / r_scaled
