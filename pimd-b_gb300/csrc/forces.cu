@@ -1204,7 +1204,7 @@ __global__ void k_bead_finish(Sys s, const double* __restrict__ part, int T, int
 
 // The whole force evaluation with the harmonic interaction of every pair
 // (FP64; harmonic_all_pairs): one block per (bead, axis) row, its sum first.
-// N = 61, P = 20: 7.5 us in place of the pair tiles' 22 and k_bead_finish's 5.
+// N = 61, P = 20: 6.4 us in place of the pair tiles' 22 and k_bead_finish's 5.
 constexpr int kRowThreads = 128;
 template <int D>
 __global__ void __launch_bounds__(kRowThreads) k_bead_finish_harmonic(Sys s, int write_phys, int add_fx) {
