@@ -517,7 +517,10 @@ __global__ void __launch_bounds__(256) k_exch_weights_rows(Sys s, int phase) {
 // N = 692 190 / 208 and 206 / 220).  Recursions alone, us, liquid and (no
 // weight zero) trap: N = 767 106 / 108 and 225 / 229, N = 1100 175 / 178 and
 // 232 / 240, N = 1500 228 / 220 and 307 / 305, N = 4096 553 / 421 and 933 / 813.
-constexpr int kTileWeightsMinN = 1280;
+// From 1000 particles on the form hardly shows in a step (liquids of 1000, 14
+// and 24 beads: 331 / 335 and 455 / 459; dipoles of 1000, 16 and 32 beads 247 /
+// 247 and 275 / 277; of 1024 and 32 beads with a cold L2 281 / 276).
+constexpr int kTileWeightsMinN = 1024;
 __global__ void __launch_bounds__(kTileThreads) k_exch_weights(Sys s, int phase, int tiles) {
     if (phase == 1 && ((volatile int*)s.xflags)[6] == 0) return;
     __shared__ double tbl[32];

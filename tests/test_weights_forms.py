@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("liquid", [False, True])
-@pytest.mark.parametrize("N", [511, 512, 513, 768, 1279, 1280, 1281])
+@pytest.mark.parametrize("N", [511, 512, 513, 768, 1023, 1024, 1025])
 def test_potentials(N, liquid):
     kw = dict(T_K=1.0, mass_amu=4.0026, pbc=True, box_ang=(N / 0.0218) ** (1 / 3)) if liquid else \
         dict(T_K=2.0, ext="harmonic", ext_p=(3.0 * MEV, 0, 0))
