@@ -1298,9 +1298,9 @@ __global__ void __launch_bounds__(kEstimatorThreads) k_exch_estimators(Sys s, in
 // that prefers a smaller one (more L1) could start only on SMs without
 // pair-tile blocks, and the pair tiles' blocks could not start beside it:
 // launched first in a step graph, the exchange would hold back part of the pair
-// kernel.  k_exch_solve_band has two blocks and SMs of its own, and
-// k_exch_estimators comes last on its stream: with them listed too, steps and
-// observables of 100 to 692 particles took the same time.
+// kernel.  k_exch_solve_band has two blocks and SMs of its own
+// (launch_solve_band), and k_exch_estimators comes last on its stream: with it
+// listed too, observables of 100 to 692 particles took the same time.
 // Attributes belong to the current device: they are set once per device (a
 // bit per device id below 64, every call above), and two host threads that
 // set them at once only repeat the same cheap calls.
@@ -1437,6 +1437,27 @@ static bool grid_estimate(const Sys& s, int phase, double* ysol, unsigned* gflag
 // one-block passes (below the multi-SM solve's size) then run alone on an SM.
 int exchange_reserved_sms(const Sys& s) { return s.N < kGridSolveMinN ? 2 : 0; }
 
+// With `alone` the launch prefers a carveout of little more than its shared
+// memory, so that its CTAs start on SMs without pair blocks (which run under the
+// largest) and the dense solve reads the weights through a large L1: started
+// under the pair blocks' carveout it keeps the small one to its end (dipoles of
+// 711 particles, 7 beads, dense weights: 295 -> 271 us a step).  Not from 768
+// particles, where the multi-SM solve waits for it (850, 32 beads: 243 -> 254).
+static void launch_solve_band(const Sys& s, int phase, double* ysol, int standalone, size_t smem, bool alone,
+                              cudaStream_t st) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(2);
+    c.blockDim = dim3(kBandThreads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at.val.sharedMemCarveout = (unsigned)((smem + 4 * 1024) * 100 / (228 * 1024) + 1);
+    c.attrs = &at;
+    c.numAttrs = alone ? 1 : 0;
+    cudaLaunchKernelEx(&c, k_exch_solve_band, s, phase, ysol, standalone);
+}
+
 int launch_exchange_recursions(const Sys& s, int exact, cudaStream_t st, double* ysol, unsigned* gflags,
                                int estimate_done) {
     exchange_carveouts();
@@ -1481,7 +1502,7 @@ int launch_exchange_recursions(const Sys& s, int exact, cudaStream_t st, double*
         if (ysol && banded_solve_fits(s)) {
             const size_t bs = std::max(banded_solve_smem(s), least);
             opt_in_smem((const void*)k_exch_solve_band, bs);
-            k_exch_solve_band<<<2, kBandThreads, bs, st>>>(s, phase, ysol, standalone);
+            launch_solve_band(s, phase, ysol, standalone, bs, standalone && least, st);
             banded = 1;
             ++n;
         }
